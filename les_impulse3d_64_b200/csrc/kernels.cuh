@@ -31,7 +31,7 @@ namespace cavity {
 // batched launch per entry.
 enum SweepKind : int { kSweepFace = 0, kSweepTile = 1, kSweepMarch = 2, kSweepPair = 3 };
 enum LaunchKind : int { kLkStepBegin = 0, kLkSweep, kLkStart, kLkResidual, kLkFinish, kLkDgemm64, kLkDgemm32, kLkTc,
-                        kLkPair };
+                        kLkPair, kLkTcPair };
 struct LaunchRecord {
     int kind, variant;
     dim3 grid;
@@ -45,6 +45,9 @@ inline thread_local int g_launch_batch = 1;
 inline thread_local int g_dgemm_tile = 0;
 // a batch's FP64 passes as three paired launches (1) or six (0); -1 outside a batch
 inline thread_local int g_batch_pairs = -1;
+// a batch's tensor-core passes as three paired launches (1: members of one size, 2: of several) or six (0); -1
+// outside a batch
+inline thread_local int g_batch_tc_pairs = -1;
 // launch a step kernel with programmatic stream serialization (see pdl_wait); inside a stream capture this makes
 // the graph edge to the previous kernel a programmatic one
 template <class... KArgs, class... Args>

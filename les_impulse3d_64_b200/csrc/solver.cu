@@ -25,6 +25,7 @@
 #include "kernels.cuh"
 #include "fdm.cuh"
 #include "tc_gemm.cuh"
+#include "tc_pair.cuh"
 #include "sweep.cuh"
 #include "sweep_march.cuh"
 #include "sweep_tile.cuh"
@@ -603,7 +604,7 @@ public:
     // the transforms' launches and the residual
     int kernels_per_step(int passes) const override { return 1 + 3 * 4 + 3 * passes * (transform_launches() + 1); }
     int transform_launches() const {
-        if (tc_fdm_) return 6;
+        if (tc_fdm_) return tc_pair_used(nx_, ny_, nz_) ? 3 : 6;
         const int f = pass_form(fdm_, form_env_ >= 0 ? form_env_ : tune_.fused);
         return f == kPassPairs ? 3 : f == kPassOneLaunch ? 1 : 6;
     }
@@ -1070,7 +1071,9 @@ private:
     }
     // the six transforms of a pass (backend.cu:801-814)
     void launch_transforms(cudaStream_t st, double* phi, cudaGraphConditionalHandle h, int use_h) {
-        if (tc_fdm_) launch_tc_pass(st, phi, h, use_h != 0);
+        if (tc_fdm_)
+            launch_tc_pass(st, tcop_, res_, rhs_, phi, reinterpret_cast<float*>(t1_), reinterpret_cast<float*>(t2_), ctrl_, h,
+                           use_h != 0, sms_);
         else {
             const int outer = g_dgemm_tile;              // a batch's choice wins over this cavity's own tuning
             if (!g_launch_record && tune_.dgemm) g_dgemm_tile = tune_.dgemm;
@@ -1078,10 +1081,6 @@ private:
                             form_env_ >= 0 ? form_env_ : tune_.fused);
             g_dgemm_tile = outer;
         }
-    }
-    void launch_tc_pass(cudaStream_t st, double* phi, cudaGraphConditionalHandle h, bool use_h) {
-        launch_tc_fdm_pass(st, tcop_, res_, rhs_, phi, reinterpret_cast<float*>(t1_), reinterpret_cast<float*>(t2_),
-                           ctrl_, h, use_h, sms_);
     }
     void launch_finish(cudaStream_t st, T* const m[3], T* const u_out[3], double* phi_out, bool step_mode, int stage,
                        bool last) {
@@ -1211,6 +1210,7 @@ private:
                 march_per_sm_ = std::max(1, march_per_sm_);
             }
             if (tc_fdm_) check(tc_transform_prepare());
+            if (tc_fdm_) check(tc_pair_prepare());
             check(pair_prepare());
             form_env_ = pass_form_from_env();
         }
@@ -1391,6 +1391,9 @@ public:
             for (const S_* s : m_) fits = fits && pair_pass_fits(s->nx_, s->ny_, s->nz_);
             const int e = pass_form_from_env();
             pairs_ = fits && (e < 0 || e == kPassPairs) ? 1 : 0;
+            bool tc_fits = true;
+            for (const S_* s : m_) tc_fits = tc_fits && tc_pair_fits(s->nx_, s->ny_, s->nz_);
+            tc_pairs_ = !tc_fits ? 0 : mixed_sizes_ ? 2 : 1;
         }
         proto_ = m_[0];
         par_ = m_[0]->par_;
@@ -1415,6 +1418,7 @@ public:
             check(cudaFuncSetAttribute(sweep_pair_batched<kTY, kTZ, S_::kPairNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)S_::PairG::template smem_bytes<T>()));
         if (f.tc_fdm_) check(tc_transform_prepare_batched());
+        if (f.tc_fdm_) check(tc_pair_prepare());
         check(pair_prepare());
         for (int S = 0; S < 2; S++) build(S);
         proto_ = nullptr;        // members may leave and be destroyed from now on
@@ -1534,7 +1538,7 @@ public:
             for (int S = 0; S < 2; S++) {
                 std::vector<LaunchRecord> rec;
                 {
-                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_);
+                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_);
                     record_member(*s, S ^ d_[slot], S);
                 }
                 const Layout& L = layout_[S];
@@ -1559,17 +1563,19 @@ public:
 
 private:
     struct RecordGuard {
-        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs) {
+        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs) {
             g_launch_record = r;
             g_launch_batch = batch;
             g_dgemm_tile = dgemm_tile;
             g_batch_pairs = pairs;
+            g_batch_tc_pairs = tc_pairs;
         }
         ~RecordGuard() {
             g_launch_record = nullptr;
             g_launch_batch = 1;
             g_dgemm_tile = 0;
             g_batch_pairs = -1;
+            g_batch_tc_pairs = -1;
         }
     };
     static size_t align256(size_t n) { return (n + 255) / 256 * 256; }
@@ -1622,7 +1628,7 @@ private:
         const size_t B = m_.size();
         std::vector<std::vector<LaunchRecord>> recs(B);
         for (size_t b = 0; b < B; b++) {
-            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_);
+            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_);
             if (m_[b]) fn(*m_[b], (int)b);
             else fn(*proto_, 0);
         }
@@ -1708,6 +1714,7 @@ private:
                              live));
             break;
         case kLkTc: launch_tc_batched(r.variant, g, items, live, (const TcTransformArgs*)d, st); break;
+        case kLkTcPair: launch_tc_pair_batched(r.variant, g, r.smem, items, live, (const TcPairArgs*)d, st); break;
         case kLkPair: launch_pair_batched(r.variant, g, items, live, (const FdmPairArgs*)d, st); break;
         default: fail("batch: unknown launch");
         }
@@ -1826,6 +1833,7 @@ private:
     Layout layout_[2];
     bool mixed_sizes_ = false;
     int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 64 cells)
+    int tc_pairs_ = 0;          // tensor-core passes as paired launches (g_batch_tc_pairs)
     int dgemm_tile_ = 0;
     std::map<std::string, size_t> item_lists_;      // work lists already in the argument buffer, by content
 };
@@ -1867,6 +1875,7 @@ static void fdm_pass_tf32(int nx, int ny, int nz, const double* const s[3], cons
     check(cudaGetDevice(&dev));
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     check(tc_transform_prepare());
+    check(tc_pair_prepare());
     std::vector<void*> owned;
     auto alloc = [&](size_t bytes) {
         void* p = nullptr;
@@ -1892,7 +1901,7 @@ static void fdm_pass_tf32(int nx, int ny, int nz, const double* const s[3], cons
     check(cudaMemcpyAsync(c, &hc, sizeof hc, cudaMemcpyHostToDevice, stream));
     control_norm_kernel<<<1, kThreads, 0, stream>>>(r, n, c);
     convert_kernel<double, float><<<blocks_for(n), kThreads, 0, stream>>>(inv_lambda, invf, n);
-    launch_tc_fdm_pass(stream, op, r, nullptr, phi, t1, t2, c, 0, false, sms);
+    launch_tc_pass(stream, op, r, nullptr, phi, t1, t2, c, 0, false, sms);
     const cudaError_t launched = cudaGetLastError();
     Control out;
     const cudaError_t copied = cudaMemcpyAsync(&out, c, sizeof out, cudaMemcpyDeviceToHost, stream);

@@ -18,9 +18,10 @@
 // 4 consecutive k; cp.async copies of the basis image) while the tensor core works on panel p.  One
 // thread issues the tcgen05.mma.cta_group::1.kind::tf32 instructions (M = 128, N = BN, K = 8) and commits each
 // panel to that stage's mbarrier.  Every mbarrier wait is bounded: on time-out the kernel records
-// kDeviceWait in the control block, frees its TMEM and returns.  Only this kernel and the staged one below
-// allocate TMEM, and their shared memory (>= 80 KB; 192 KB for the staged kernel's 128 columns) keeps at most two
-// CTAs of <= 64 columns, or one of 128, on an SM, below its 512 columns.
+// kDeviceWait in the control block, frees its TMEM and returns.  This kernel and the staged one below run a pass where
+// an axis has more than 256 cells (else tc_pair.cuh runs it as three launches).  Their shared memory (>= 80 KB; 192 KB
+// for the staged kernel's 128 columns) keeps at most two CTAs of <= 64 columns, or one of 128, on an SM, below its 512
+// columns.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -833,17 +834,21 @@ template <int BN> inline void launch_tc_bn(cudaStream_t st, const TcTransformArg
 }
 // variant code of a recorded launch: tile width, field-is-A, fp64 field
 inline int tc_variant(int bn, const TcTransformArgs& g) { return bn | (g.field_is_a ? 1 << 8 : 0) | (g.field64 ? 1 << 9 : 0); }
-// The staged kernel (tc2_transform_body) for a single cavity's launch whose 128 x 128 tiles fit on the SMs at
-// once (one CTA per SM): there its deeper prefetch shortens the one CTA chain the launch lasts (C3 pass 84 against
-// 88 us).  With more tiles than SMs, and in batches, the register-pipelined kernel, whose two CTAs per SM overlap
-// each other's latencies (C6 pass 860 against 872 us).  CAVITY_TC_KERNEL=staged or =panel forces either.
-inline bool tc_use_staged(const TcTransformArgs& g, int batch, int sms) {
+// CAVITY_TC_KERNEL=staged or =panel: the pass as six launches of that kernel (1, 0; -1: not set)
+inline int tc_kernel_forced() {
     static const int forced = [] {
         const char* e = std::getenv("CAVITY_TC_KERNEL");
         if (!e) return -1;
         return std::string(e) == "staged" ? 1 : std::string(e) == "panel" ? 0 : -1;
     }();
-    if (forced >= 0) return forced == 1;
+    return forced;
+}
+// The staged kernel (tc2_transform_body) for a single cavity's launch whose 128 x 128 tiles fit on the SMs at
+// once (one CTA per SM): there its deeper prefetch shortens the one CTA chain the launch lasts (C3 pass 84 against
+// 88 us).  With more tiles than SMs, and in batches, the register-pipelined kernel, whose two CTAs per SM overlap
+// each other's latencies (C6 pass 860 against 872 us).  CAVITY_TC_KERNEL=staged or =panel forces either.
+inline bool tc_use_staged(const TcTransformArgs& g, int batch, int sms) {
+    if (tc_kernel_forced() >= 0) return tc_kernel_forced() == 1;
     if (g_launch_record) return false;
     const long long tiles = (long long)((g.N + kTc2BN - 1) / kTc2BN) * ((g.M + kTcRows - 1) / kTcRows) * batch;
     return tiles <= sms;
