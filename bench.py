@@ -238,15 +238,16 @@ def transforms_roofline(settings, ms_per_pass, tc, peak_gbs, launches=6):
     bytes against HBM.  Six launches move 16 B per cell per transform (an 8-byte read and write; the first reads
     the FP64 residual, the last updates the FP64 potential) plus 8 B of 1/lambda; the three paired launches of
     the FP64 pass (`launches` = 3) keep every second intermediate on chip: 8 B in and out each, 8 B of 1/lambda
-    and 8 B of the potential read."""
+    and 8 B of the potential read; the mixed form's keep it in TMEM and move 4 B intermediates and 1/lambda."""
     nx, ny, nz = settings['nx'], settings['ny'], settings['nz']
     cells = nx * ny * nz
     flops = 4.0 * (nx + ny + nz) * cells * (3 if tc else 1)
-    paired = not tc and launches == 3
-    nbytes = (3 * 16 + 16 if paired else 6 * 16 + 8) * cells
+    paired = launches == 3
+    nbytes = (44 if tc and paired else 3 * 16 + 16 if paired else 6 * 16 + 8) * cells
     s = ms_per_pass / 1e3
     peak = gemm_peak_tflops('tf32' if tc else 'fp64')
-    name = ('tc2_transform_kernel / tc_transform_kernel (tcgen05 3xTF32)' if tc else
+    name = ('tc_pair_kernel (tcgen05 3xTF32, two transforms per launch)' if tc and paired else
+            'tc2_transform_kernel / tc_transform_kernel (tcgen05 3xTF32)' if tc else
             'pair_xy/pair_z/pair_yx_kernel (FP64 DMMA, two transforms per launch)' if paired else
             'dgemm_mma_kernel (FP64 DMMA)')
     return {'kernel': name, 'launches_per_pass': launches,
@@ -426,6 +427,10 @@ def run_ours(args, ranks):
     # the other stencil kernels of the step, timed by events in the same graph (their launches in all stages)
     cell_kernels = {}
     for name, nbytes in cell_kernel_bytes(s, field_bytes).items():
+        if ktimes['guess_residual'] == 0.0:        # one launch forms the guess and its residual: nothing is read back
+            if name == 'guess_residual':
+                continue
+            nbytes += 8 * cells if name == 'projection_start' else 0
         launch_s = ranks.max(ktimes[name]) / 1e3 / 3
         gbs = nbytes / launch_s / 1e9 if launch_s > 0 else None
         cell_kernels[name] = {'ms_per_launch': launch_s * 1e3, 'bytes_per_launch': nbytes, 'achieved_gbs': gbs,

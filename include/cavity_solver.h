@@ -115,8 +115,8 @@ int cavity_time_steps(CavitySolver* s, int warmup, int steps, int flush_l2, floa
  * the size rule), and the step time in milliseconds. */
 int cavity_autotune(CavitySolver* s, int steps, int* march_chunks, int* dgemm_tile, int* fused_pass, float* ms_per_step);
 /* After cavity_time_steps: ms[5] receives the mean device time per timed step (milliseconds, all three stages)
- * of the momentum sweeps, the projection starts, the residuals of their warm-start guesses, the finishes, and
- * the six transforms of each stage's first pressure pass.  No counterpart in the reference. */
+ * of the momentum sweeps, the projection starts, the residuals of their warm-start guesses (0 where the start forms
+ * them itself), the finishes, and the six transforms of each stage's first pressure pass.  No counterpart in the reference. */
 int cavity_kernel_times(CavitySolver* s, double* ms);
 /* The generalised eigenbasis of one axis's pressure operator, K S = W S diag(lambda) with S^T W S = I, for the grid
  * that `config` describes along `axis` (0 x, 1 y, 2 z): lambda[n] (the constant mode set to 0) and the row-major

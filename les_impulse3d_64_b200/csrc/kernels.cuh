@@ -48,6 +48,8 @@ inline thread_local int g_batch_pairs = -1;
 // a batch's tensor-core passes as three paired launches (1: members of one size, 2: of several) or six (0); -1
 // outside a batch
 inline thread_local int g_batch_tc_pairs = -1;
+// whether a batch's projections start in one launch with the residual of the guess (fused_start_kernel)
+inline thread_local bool g_batch_fused_start = false;
 // launch a step kernel with programmatic stream serialization (see pdl_wait); inside a stream capture this makes
 // the graph edge to the previous kernel a programmatic one
 template <class... KArgs, class... Args>
@@ -405,6 +407,7 @@ template <class T> struct StartArgs {
     double* rhs;
     double* res;
     double* guess;              // the starting potential (the buffer the solve refines)
+    int tiles_x;                // fused start: tiles along x; blocks' x runs over the tiles of a plane
     // step only (base == nullptr: a plain projection)
     const double* phi_state;    // stage 0: state potential
     double* phi0;               // stage 0 writes, stages 1, 2 read
@@ -588,6 +591,206 @@ __global__ void __launch_bounds__(kThreads, kColumnBlocks) projection_start_batc
     if (cav < 0) return;
     load_args(a, args + cav);
     projection_start_body(a, k);
+}
+
+// The start of a step's projection and the residual of its guess in one launch, for small grids: a block walks
+// a kStartX x kStartY tile of columns up a chunk of z-layers.  A layer's guess is evaluated once per cell, and once more
+// on the tile's rim, into one of two planes in shared memory, from which the layer's residual takes its x- and
+// y-neighbours; the guess below, at and above a cell's layer stays in registers.  The values are those of the two
+// launches, bit for bit; only the sums' grouping differs.
+// It saves a launch and a grid-wide reduction before every solve where launches are latency (32 x 32 x 8: the two took
+// 67 us of a step's 173, this one 39; 64^3: 81 and 50), but a barrier per layer and the rim cost more than they save
+// where the walks are bound by HBM (256^3: 871 us as two launches, 1,050 as one; a batch of 7 x 64^3: 158 and 234):
+// see fused_start in the solver.  Compiled for two blocks per SM: for four it spilled (64^3: 66 us).
+constexpr int kStartX = 32, kStartY = 8, kStartBlocks = 2;
+template <class T>
+__device__ void fused_start_body(const StartArgs<T>& a, const Blk& k) {
+    pdl_launch_dependents();
+    pdl_wait();
+    static_assert(kStartX == 32 && kStartX * kStartY == kThreads, "a warp is a row of the tile");
+    constexpr int W = kStartX + 2, H = kStartY + 2, RIM = 2 * kStartX + 2 * kStartY;
+    __shared__ double plane[2][H * W];
+    Control* c = a.c;
+    const Params& p = a.p;
+    const int err = c->error;
+    const StageConst sc = stage_const(a.stage, c);
+    int b1 = -1, b2 = -1;
+    double c1 = 0, c2 = 0;
+    guess_coefficients(p, c, sc.tau, sc.b * c->dt, b1, c1, b2, c2);
+    Vec<3> acc;                                   // rhs^2, residual^2, guess
+    acc.v[0] = acc.v[1] = acc.v[2] = 0.0;
+    const int nx = p.nx, ny = p.ny, nz = p.nz, sz = nx * ny;
+    const int zc = (nz + (int)k.ny - 1) / (int)k.ny, z0 = (int)k.y * zc, z1 = min(nz, z0 + zc);
+    if (!err && z0 < z1) {
+        const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+        const int x0 = (int)(k.x % a.tiles_x) * kStartX, y0 = (int)(k.x / a.tiles_x) * kStartY;
+        const int x = x0 + tx, y = y0 + ty;
+        const bool live = x < nx && y < ny;
+        const int su = (nx + 1) * ny, sv = nx * (ny + 1);             // layer strides of the u and v faces
+        // this thread's rim cell, if it has one inside the box
+        int rx = -1, ry = -1, ro = 0;
+        if (t < kStartX) { rx = x0 + t; ry = y0 - 1; ro = t + 1; }
+        else if (t < 2 * kStartX) { rx = x0 + t - kStartX; ry = y0 + kStartY; ro = (H - 1) * W + t - kStartX + 1; }
+        else if (t < RIM) {
+            const int e = t - 2 * kStartX, r = e % kStartY, right = e / kStartY;
+            rx = right ? x0 + kStartX : x0 - 1;
+            ry = y0 + r;
+            ro = (r + 1) * W + (right ? W - 1 : 0);
+        }
+        const bool rim = rx >= 0 && rx < nx && ry >= 0 && ry < ny;
+        const int own = (ty + 1) * W + tx + 1, cell = x + nx * y, rcell = rx + nx * ry;
+        const int stage = a.stage;
+        struct Pot { double ph, p0, h1, h2; };
+        auto potentials = [&](int j) {            // what the guess of cell j is made of
+            Pot v;
+            v.p0 = v.h1 = v.h2 = 0.0;
+            v.ph = __ldg((stage == 0 ? a.phi_state : a.phi_cur) + j);
+            if (stage != 0) v.p0 = __ldg(a.phi0 + j);
+            if (b1 >= 0) v.h1 = __ldg(a.hist[b1] + j);
+            if (b2 >= 0) v.h2 = __ldg(a.hist[b2] + j);
+            return v;
+        };
+        // base and guess (backend.cu:922-928, 857-873)
+        auto base_of = [&](const Pot& v) { return stage == 0 ? sc.b * (p.reinit_r * v.ph) : sc.a0 * v.p0 + sc.b * v.ph; };
+        auto guess_of = [&](const Pot& v, double base) {
+            if (b1 < 0) return base;
+            const double e = b2 >= 0 ? c1 * v.h1 + c2 * v.h2 : c1 * v.h1;
+            return e + base;
+        };
+        const double dx = live ? a.g.dw[X][x] : 0.0, dy = live ? a.g.dw[Y][y] : 0.0;
+        const bool xl = x > 0, xh = x + 1 < nx, yl = y > 0, yh = y + 1 < ny;
+        const double ixl = live ? a.g.dinv_sp[X][x] : 0.0, ixh = live ? a.g.dinv_sp[X][x + 1] : 0.0;
+        const double iyl = live ? a.g.dinv_sp[Y][y] : 0.0, iyh = live ? a.g.dinv_sp[Y][y + 1] : 0.0;
+        // the loads of a layer, issued one layer ahead of their use
+        struct Faces { T mx0, mx1, my0, my1, mz1; double dz; };
+        auto faces = [&](int z) {
+            const int iu = z * su + x + (nx + 1) * y, iv = z * sv + cell;
+            Faces f;
+            f.mx0 = __ldg(a.m[X] + iu);
+            f.mx1 = __ldg(a.m[X] + iu + 1);
+            f.my0 = __ldg(a.m[Y] + iv);
+            f.my1 = __ldg(a.m[Y] + iv + nx);
+            f.mz1 = __ldg(a.m[Z] + (z + 1) * sz + cell);
+            f.dz = __ldg(a.g.dw[Z] + z);
+            return f;
+        };
+        double below = 0.0, cc = 0.0, base = 0.0, ph = 0.0;      // the guess below and at layer z; base and potential there
+        Pot above = {}, rabove = {};                             // layer z + 1, here and at the rim cell
+        Faces next = {};
+        T wlo = T(0);
+        if (live) {
+            next = faces(z0);
+            wlo = __ldg(a.m[Z] + z0 * sz + cell);                // m_z on the first cell's lower face
+            const Pot v = potentials(z0 * sz + cell);
+            if (z0 > 0) {
+                const Pot u = potentials((z0 - 1) * sz + cell);
+                below = guess_of(u, base_of(u));
+            }
+            if (z0 + 1 < nz) above = potentials((z0 + 1) * sz + cell);
+            ph = v.ph;
+            base = base_of(v);
+            cc = guess_of(v, base);
+            plane[0][own] = cc;
+        }
+        if (rim) {
+            const Pot v = potentials(z0 * sz + rcell);
+            if (z0 + 1 < z1) rabove = potentials((z0 + 1) * sz + rcell);
+            plane[0][ro] = guess_of(v, base_of(v));
+        }
+        for (int z = z0; z < z1; z++) {
+            __syncthreads();                       // layer z's plane is complete, the other one no longer read
+            const double* q = plane[(z - z0) & 1];
+            double* qn = plane[(z - z0 + 1) & 1];
+            const bool zh = z + 1 < nz;
+            if (rim && z + 1 < z1) {
+                const Pot v = rabove;
+                if (z + 2 < z1) rabove = potentials((z + 2) * sz + rcell);
+                qn[ro] = guess_of(v, base_of(v));
+            }
+            if (!live) continue;
+            const Faces f = next;
+            if (z + 1 < z1) next = faces(z + 1);
+            double nbase = 0.0, ng = 0.0, nph = 0.0;
+            if (zh) {
+                const Pot v = above;
+                if (z + 2 < nz && z + 1 < z1) above = potentials((z + 2) * sz + cell);
+                nph = v.ph;
+                nbase = base_of(v);
+                ng = guess_of(v, nbase);
+                if (z + 1 < z1) qn[own] = ng;
+            }
+            const double dz = f.dz;
+            const double rhs = ((double)f.mx1 - (double)f.mx0) * (dy * dz) + ((double)f.my1 - (double)f.my0) * (dx * dz) +
+                               ((double)f.mz1 - (double)wlo) * (dx * dy);
+            wlo = f.mz1;
+            const int i = z * sz + cell;
+            a.rhs[i] = rhs;
+            acc.v[0] += rhs * rhs;
+            if (stage == 0) a.phi0[i] = p.reinit_r * ph;
+            a.base[i] = base;
+            a.guess[i] = cc;
+            double s = 0.0;                        // L guess, as the residual after a pass (residual_body)
+            if (xh) s += (dy * dz) * (q[own + 1] - cc) * ixh;
+            if (xl) s -= (dy * dz) * (cc - q[own - 1]) * ixl;
+            if (yh) s += (dx * dz) * (q[own + W] - cc) * iyh;
+            if (yl) s -= (dx * dz) * (cc - q[own - W]) * iyl;
+            if (zh) s += (dx * dy) * (ng - cc) * __ldg(a.g.dinv_sp[Z] + z + 1);
+            if (z > 0) s -= (dx * dy) * (cc - below) * __ldg(a.g.dinv_sp[Z] + z);
+            const double r = rhs - s;
+            a.res[i] = r;
+            acc.v[1] += r * r;
+            acc.v[2] += cc;
+            below = cc;
+            cc = ng;
+            base = nbase;
+            ph = nph;
+        }
+    }
+    const Vec<3> blk = block_reduce<3, false>(acc);
+    if (publish_partials(blk, a.partial, &c->counter[kCntDiv], k)) {
+        const Vec<3> tot = final_reduce<3, false>(a.partial, k);
+        if (threadIdx.x == 0) {
+            c->counter[kCntDiv] = 0;
+            c->passes = 0;
+            c->phi_passes = 0;
+            c->reset_phi = 0;
+            c->zero_rhs = 0;
+            if (err) { set_loop(c, a.handle, a.use_handle, 0); return; }
+            c->rhs_norm2 = tot.v[0];
+            c->rhs_norm = sqrt(tot.v[0]);
+            if (!isfinite(c->rhs_norm)) { c->error = kRhsNaN; set_loop(c, a.handle, a.use_handle, 0); return; }
+            if (c->rhs_norm == 0.0) {                         // backend.cu:821: phi = 0
+                c->zero_rhs = 1;
+                c->reset_phi = 1;
+                c->phi_rel = 0.0;
+                c->phi_sum = 0.0;
+                c->rel = 0.0;
+                set_loop(c, a.handle, a.use_handle, 0);
+                return;
+            }
+            // the guess is kept unless it is no better than zero (backend.cu:825-831)
+            double rel = sqrt(tot.v[1]) / c->rhs_norm;
+            c->res_norm2 = tot.v[1];
+            c->use_rhs = 0;
+            c->phi_sum = tot.v[2];
+            if (rel >= 1.0) { rel = 1.0; c->use_rhs = 1; c->reset_phi = 1; c->phi_sum = 0.0; }
+            c->rel = rel;
+            decide_loop(p, c, a.handle, a.use_handle);
+        }
+    }
+}
+template <class T>
+__global__ void __launch_bounds__(kThreads, kStartBlocks) fused_start_kernel(StartArgs<T> a) {
+    fused_start_body(a, real_blk());
+}
+template <class T>
+__global__ void __launch_bounds__(kThreads, kStartBlocks) fused_start_batched(const StartArgs<T>* args, const BatchItem* items, const int* live) {
+    __shared__ StartArgs<T> a;
+    int cav;
+    const Blk k = item_blk(items, live, cav);
+    if (cav < 0) return;
+    load_args(a, args + cav);
+    fused_start_body(a, k);
 }
 
 // ------------------------------------------------------------------------------------------ residual

@@ -599,10 +599,11 @@ public:
     }
     long long device_bytes() const override { return arena_.bytes(); }
 
-    // step begin; per stage the sweep, the projection start, the residual of its guess and the finish; 7 per pass
-    // step begin, then per stage the sweep, the projection start, its guess's residual and the finish, and per pass
-    // the transforms' launches and the residual
-    int kernels_per_step(int passes) const override { return 1 + 3 * 4 + 3 * passes * (transform_launches() + 1); }
+    // step begin, then per stage the sweep, the projection start, its guess's residual (one launch with the start where
+    // fused) and the finish, and per pass the transforms' launches and the residual
+    int kernels_per_step(int passes) const override {
+        return 1 + 3 * (fused_start() ? 3 : 4) + 3 * passes * (transform_launches() + 1);
+    }
     int transform_launches() const {
         if (tc_fdm_) return tc_pair_used(nx_, ny_, nz_) ? 3 : 6;
         const int f = pass_form(fdm_, form_env_ >= 0 ? form_env_ : tune_.fused);
@@ -639,6 +640,7 @@ public:
                     continue;
                 }
                 for (int kind = 0; kind < kNumTimed; kind++) {
+                    if (kind == kTkGuessResidual && fused_start()) continue;      // timed with the start
                     float tot = 0, t;
                     for (int s = 0; s < 3; s++) {
                         check(cudaEventElapsedTime(&t, kev(kind, s)[0], kev(kind, s)[1]));
@@ -794,7 +796,7 @@ private:
         t2_ = arena_.alloc<double>(n_cell_);
         inv_lambda_ = arena_.alloc<double>(n_cell_);
         // the grid-stride kernels' blocks, or the column kernels' plane blocks x z-chunks (at most one chunk per layer)
-        partial_blocks_ = std::max((long long)blocks_for(std::max(max_face_, n_cell_)),
+        partial_blocks_ = std::max(std::max((long long)blocks_for(std::max(max_face_, n_cell_)), start_tiles() * nz_),
                                    (long long)blocks_for((long long)nx_ * ny_) * nz_) + 8;
         int sms = 148, dev = 0;
         check(cudaGetDevice(&dev));
@@ -961,9 +963,21 @@ private:
     // for the launch (all cavities of a batch together) to fill the device `per_sm` blocks deep in one wave, or
     // about four waves when the plane blocks alone exceed one
     dim3 column_grid(int per_sm, int per_thread = 1) const {
-        const long long bpp = blocks_for((long long)nx_ * ny_ / per_thread);
+        return chunked_grid(blocks_for((long long)nx_ * ny_ / per_thread), per_sm);
+    }
+    // tiles of a plane of the fused projection start
+    long long start_tiles() const {
+        return (long long)((nx_ + kStartX - 1) / kStartX) * ((ny_ + kStartY - 1) / kStartY);
+    }
+    // The projection start and the residual of its guess as one launch: for at most 2^18 cells in all (a batch's members
+    // together).  Measured against two launches (us per step): 32 x 32 x 8 161 / 173, 32^3 174 / 188, 50 x 50 x 37 201 /
+    // 215, 64^3 272 / 282, 64 x 64 x 128 394 / 402; 100 x 100 x 75 FP64 897 / 894, 128^3 960 / 939, 7 x 64^3 997 / 920.
+    // Its chunks do not depend on the batch, so that a member's sums are grouped as those of the cavity alone.
+    static constexpr long long kFusedStartCells = 1LL << 18;
+    bool fused_start() const { return g_launch_record ? g_batch_fused_start : n_cell_ <= kFusedStartCells; }
+    dim3 chunked_grid(long long bpp, int per_sm, int cavities = 0) const {
         const long long want = (long long)sms_ * std::max(per_sm, 1);
-        const long long cav = std::max(g_launch_batch, 1);
+        const long long cav = cavities > 0 ? cavities : std::max(g_launch_batch, 1);
         long long chunks = want / (bpp * cav);
         // a launch that holds more plane blocks than fit at once (a large batch): chunks for about four waves, so
         // that the last, partial wave is a small share of the launch
@@ -1023,7 +1037,7 @@ private:
     }
     // rhs, starting potential and its residual, start-of-solve decisions (backend.cu:816-831)
     // use_h: 0 no graph loop, 1 this solver's own loop, 2 a loop shared by a batch (see set_loop); `between` runs
-    // between the start kernel and the residual of the guess (timing events)
+    // between the start kernel and the residual of the guess (timing events) where they are two launches
     void launch_start(cudaStream_t st, T* const m[3], bool step_mode, int stage, int S, int cur,
                       cudaGraphConditionalHandle h, int use_h, const std::function<void()>& between = {}) {
         StartArgs<T> a;
@@ -1043,6 +1057,13 @@ private:
         a.partial = partial_;
         a.handle = h;
         a.use_handle = use_h;
+        if (step_mode && fused_start()) {
+            a.tiles_x = (nx_ + kStartX - 1) / kStartX;
+            const dim3 grid = chunked_grid(start_tiles(), kStartBlocks, 1);
+            if (!record_launch(kLkStart, 1, grid, 0, a))
+                check(launch_pdl(fused_start_kernel<T>, grid, dim3(kThreads), 0, st, a));
+            return;
+        }
         const dim3 grid = column_grid(start_per_sm_);
         if (!record_launch(kLkStart, 0, grid, 0, a))
             check(launch_pdl(projection_start_kernel<T>, grid, dim3(kThreads), 0, st, a));
@@ -1152,10 +1173,10 @@ private:
             launch_momentum(stream_, stage, S, in, out);
             if (timing) mark(kev(kTkSweep, stage)[1]);
             double* phi = praw_;          // the solve works here; finish writes PHI_[out]
-            // with timing: events around the projection start and around the residual of its guess
+            // with timing: events around the projection start and around the residual of its guess (one launch where fused)
             std::function<void()> between;
-            if (timing) {
-                mark(kev(kTkStart, stage)[0]);
+            if (timing) mark(kev(kTkStart, stage)[0]);
+            if (timing && !fused_start()) {
                 between = [&, stage] {
                     mark(kev(kTkStart, stage)[1]);
                     mark(kev(kTkGuessResidual, stage)[0]);
@@ -1163,7 +1184,7 @@ private:
             }
             if (eager) {
                 launch_start(stream_, M_[out], true, stage, S, cur, 0, 0, between);
-                if (timing) mark(kev(kTkGuessResidual, stage)[1]);
+                if (timing) mark(kev(fused_start() ? kTkStart : kTkGuessResidual, stage)[1]);
                 pull_control();
                 for (int pass = 0; hc_.cond && !hc_.error; pass++) {
                     if (timing && pass == 0) mark(kev(kTkTransforms, stage)[0]);
@@ -1175,7 +1196,7 @@ private:
             } else {
                 captured_loop([&](cudaGraphConditionalHandle h) {
                     launch_start(stream_, M_[out], true, stage, S, cur, h, 1, between);
-                    if (timing) mark(kev(kTkGuessResidual, stage)[1]);
+                    if (timing) mark(kev(fused_start() ? kTkStart : kTkGuessResidual, stage)[1]);
                 }, phi, timing ? kev(kTkTransforms, stage)[0] : nullptr, timing ? kev(kTkTransforms, stage)[1] : nullptr);
             }
             if (timing) mark(kev(kTkFinish, stage)[0]);
@@ -1394,6 +1415,9 @@ public:
             bool tc_fits = true;
             for (const S_* s : m_) tc_fits = tc_fits && tc_pair_fits(s->nx_, s->ny_, s->nz_);
             tc_pairs_ = !tc_fits ? 0 : mixed_sizes_ ? 2 : 1;
+            long long cells = (long long)(capacity - (int)m_.size()) * f.n_cell_;
+            for (const S_* s : m_) cells += s->n_cell_;
+            fused_start_ = cells <= S_::kFusedStartCells;
         }
         proto_ = m_[0];
         par_ = m_[0]->par_;
@@ -1538,7 +1562,7 @@ public:
             for (int S = 0; S < 2; S++) {
                 std::vector<LaunchRecord> rec;
                 {
-                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_);
+                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_);
                     record_member(*s, S ^ d_[slot], S);
                 }
                 const Layout& L = layout_[S];
@@ -1563,12 +1587,13 @@ public:
 
 private:
     struct RecordGuard {
-        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs) {
+        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs, bool fused_start) {
             g_launch_record = r;
             g_launch_batch = batch;
             g_dgemm_tile = dgemm_tile;
             g_batch_pairs = pairs;
             g_batch_tc_pairs = tc_pairs;
+            g_batch_fused_start = fused_start;
         }
         ~RecordGuard() {
             g_launch_record = nullptr;
@@ -1576,6 +1601,7 @@ private:
             g_dgemm_tile = 0;
             g_batch_pairs = -1;
             g_batch_tc_pairs = -1;
+            g_batch_fused_start = false;
         }
     };
     static size_t align256(size_t n) { return (n + 255) / 256 * 256; }
@@ -1628,7 +1654,7 @@ private:
         const size_t B = m_.size();
         std::vector<std::vector<LaunchRecord>> recs(B);
         for (size_t b = 0; b < B; b++) {
-            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_);
+            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_);
             if (m_[b]) fn(*m_[b], (int)b);
             else fn(*proto_, 0);
         }
@@ -1697,7 +1723,10 @@ private:
                                  (const MomentumArgs<T>*)d, items, live));
             break;
         case kLkStart:
-            check(launch_pdl(projection_start_batched<T>, g, dim3(kThreads), 0, st, (const StartArgs<T>*)d, items, live));
+            if (r.variant == 1)
+                check(launch_pdl(fused_start_batched<T>, g, dim3(kThreads), 0, st, (const StartArgs<T>*)d, items, live));
+            else
+                check(launch_pdl(projection_start_batched<T>, g, dim3(kThreads), 0, st, (const StartArgs<T>*)d, items, live));
             break;
         case kLkResidual:
             check(launch_pdl(residual_batched, g, dim3(kThreads), 0, st, (const ResidualArgs*)d, items, live));
@@ -1833,6 +1862,7 @@ private:
     Layout layout_[2];
     bool mixed_sizes_ = false;
     int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 64 cells)
+    bool fused_start_ = false;  // projection starts with their guesses' residuals in one launch
     int tc_pairs_ = 0;          // tensor-core passes as paired launches (g_batch_tc_pairs)
     int dgemm_tile_ = 0;
     std::map<std::string, size_t> item_lists_;      // work lists already in the argument buffer, by content
@@ -1856,7 +1886,8 @@ static long long estimate_bytes(const CavityConfig& c, int precision) {
                                                     cavity::basis_image_floats((int)nz, (int)nz))
                              : 0;
     return 7 * faces * fb + 16 * cells * 8 + 2 * 8 * maxface + 4 * std::max(maxface, 2 * cells) +
-           2 * 8 * (nx * nx + ny * ny + nz * nz) + 64 * (maxface / 256 + 8) + tc + (1 << 20);
+           2 * 8 * (nx * nx + ny * ny + nz * nz) +
+           64 * (std::max(maxface / 256, (nx + kStartX - 1) / kStartX * ((ny + kStartY - 1) / kStartY) * nz) + 8) + tc + (1 << 20);
 }
 
 // One FDM pass of the mixed form on the tensor cores on caller-provided device arrays, with the reference's
