@@ -45,7 +45,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // flight at once (cp.async, zero-filled outside the matrices; two doubles per copy where rows allow).
 template <int BM, int BN, int WARPS_M, int WARPS_N, int KC>
 __device__ void dgemm_mma_body(const GemmArgs<double>& g, const Blk& blk, bool first) {
-    pdl_launch_dependents();
     pdl_wait();
     constexpr int NT = WARPS_M * WARPS_N * 32;
     constexpr int WTM = BM / WARPS_M, WTN = BN / WARPS_N;     // warp tile
@@ -116,6 +115,7 @@ __device__ void dgemm_mma_body(const GemmArgs<double>& g, const Blk& blk, bool f
         }
         __syncthreads();
     }
+    pdl_launch_dependents();
     const int reset = c->reset_phi;
 #pragma unroll
     for (int i = 0; i < FM; i++) {
@@ -240,7 +240,6 @@ __device__ __forceinline__ void pair_warp_mma(double (&acc)[FM][FN][2], const do
 // Each kernel issues the copies that do not depend on the control block before reading it, so that their
 // latencies overlap; a block with nothing to do waits for its copies to land before it exits.
 __device__ __forceinline__ void pair_begin(const FdmPairArgs& a, bool first, bool clear) {
-    pdl_launch_dependents();
     pdl_wait();
     if (clear && a.clear_condition && threadIdx.x == 0 && first) cudaGraphSetConditional(a.handle, 0u);
 }
@@ -306,6 +305,7 @@ __device__ void pair_xy_body(const FdmPairArgs& a, const Blk& blk, bool first) {
         }
         const int y = m0 + fr;
         if (m0 < my) {
+            if (z + 1 == z1) pdl_launch_dependents();
             pair_warp_mma<1, FN>(acc, A2, kPairPitch, C1, PW, ky, m0, 0);
             if (y < ny) {
                 double* t = a.t + ((long long)z * ny + y) * nx;
@@ -377,6 +377,7 @@ __device__ void pair_z_body(const FdmPairArgs& a, const Blk& blk, bool first) {
         }
         const int z = m0 + fr;
         if (m0 < mz) {
+            if (b + 1 == b1) pdl_launch_dependents();
             pair_warp_mma<1, FN>(acc, A2, kPairPitch, C1, PW, kz, m0, 0);
             if (z < nz) {
                 double* t = a.t + (long long)z * plane;
@@ -450,6 +451,7 @@ __device__ void pair_yx_body(const FdmPairArgs& a, const Blk& blk, bool first) {
             cp_async_commit();
         }
         if (active) {
+            if (z + 1 == z1) pdl_launch_dependents();
             pair_warp_mma<1, FN>(acc, C1, kPairPitch, B2, kPairPitch, kx, m0, n0);
             if (y < ny) {
 #pragma unroll

@@ -2,10 +2,10 @@
 //
 // One `Solver<T>` owns one cavity: its fields in HBM, a CUDA stream, and two instantiated CUDA graphs of a
 // whole time step (one per state parity, since the step writes the next state into the other buffer set).
-// A step is one graph launch: 1 + 3 x 4 kernels plus, per stage, a conditional while-node whose body is one
-// pressure pass (6 transform launches and a residual); the residual's last block decides on the device
-// whether another pass runs.  The host waits once per step, to read the 200-byte control block that holds
-// the clock, the report and any error.
+// A step is one graph launch: a chain of kernels with one pressure pass per stage (two on the tensor cores), the last
+// block of whose residual decides on the device whether the solve is done; a solve that needs more passes is finished
+// by the host (Solver::settle).  The host waits once per step, to read the control block that holds the clock, the
+// report and any error.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -285,7 +285,7 @@ public:
             if (eager_) enqueue_step(par_, false, true);
             else check(cudaGraphLaunch(exec_[par_], stream_));
             // the parity flips only when the step succeeds; sync() checks that for the queued steps
-            pending_.push_back(par_);
+            pending_.push_back({par_});
             par_ ^= 1;
             char* d = static_cast<char*>(tail_dev_);
             step_tail_kernel<T><<<1, 32, 0, stream_>>>(out_args(), probe_cells_, c_.n_probes,
@@ -295,20 +295,19 @@ public:
         tail_queued_ = true;
     }
     void sync(CavityReport* r) override {
-        check(cudaStreamSynchronize(stream_));
-        if (tail_queued_) std::memcpy(&hc_, tail_control(), sizeof hc_);      // written by the last step's tail
-        else pull_control();
+        settle();
         const bool tail = tail_queued_;
         tail_queued_ = false;
         probes_fresh_ = false;
         const size_t queued = pending_.size();
-        const std::vector<int> pending_copy = pending_;
+        const std::vector<Pending> pending_copy = pending_;
         pending_.clear();
+        batch_pending_ = false;
         if (hc_.error) {
             // steps before the failed one committed; the failed step left the state buffers of its parity
             // untouched and every later queued step skipped its work
             const long long ok = hc_.steps - steps_before_;
-            par_ = (ok >= 0 && ok < (long long)queued) ? pending_copy[ok] : par_;
+            par_ = (ok >= 0 && ok < (long long)queued) ? pending_copy[ok].par : par_;
             const int code = hc_.error;
             hc_.error = kOk;
             push_control();
@@ -319,6 +318,48 @@ public:
         probes_fresh_ = tail && !pending_copy.empty();
         if (r) report(r);
     }
+    // Wait for the queued steps and read the control block.  A step's graph runs one pressure pass per solve (two on the
+    // tensor cores, whose FP32 transforms usually take a second): a conditional while-node for the rare further pass cost
+    // 9 us per solve even when it ran nothing, the breaks in the chain of programmatic launches included (a step of
+    // 32 x 32 x 8 cells 173 us with them, 146 without; 64^3 282 and 256).  A solve that needs more stalls: the rest of the
+    // queued work returns at once, the state it reads being untouched, and the host finishes that step and the queued
+    // ones after it here, pass by pass.  From then on the cavity's graphs have the while-nodes (loops_).
+    void settle() {
+        check(cudaStreamSynchronize(stream_));
+        if (tail_queued_) std::memcpy(&hc_, tail_control(), sizeof hc_);      // written by the last step's tail
+        else pull_control();
+        if (hc_.error == kStalled) resume_stalled();
+    }
+    // before an operation that reads the state while steps may be queued (a batch's steps are settled by its sync)
+    void settle_queued() {
+        if (!pending_.empty() && !batch_pending_) settle();
+    }
+    void resume_stalled() {
+        loops_ = true;
+        drop_graphs();
+        tail_queued_ = false;
+        const long long done = hc_.steps - steps_before_;
+        hc_.error = kOk;
+        push_control();
+        for (size_t k = (size_t)std::max(done, 0LL); k < pending_.size(); k++) {
+            const Pending q = pending_[k];
+            if ((long long)k == done) {
+                const int stage = hc_.stage;
+                continue_passes(false, stage);
+                finish_stage(q.par, stage, false, true);
+                for (int s = stage + 1; s < 3; s++) enqueue_stage(q.par, s, false, true);
+            } else {
+                enqueue_step(q.par, false, true);
+            }
+            pull_control();
+            if (hc_.error) return;
+            if (q.ring >= 0)
+                probes_kernel<T><<<1, 32, 0, stream_>>>(out_args(q.par ^ 1), probe_cells_, c_.n_probes,
+                                                        ring_dev_ + (size_t)q.ring * 2 * c_.n_probes);
+            if (q.statistics) launch_statistics(q.par ^ 1);
+        }
+        check(cudaStreamSynchronize(stream_));
+    }
     void report(CavityReport* r) override {
         r->steps = hc_.steps; r->time = hc_.t; r->dt = hc_.last_dt; r->cfl = hc_.last_cfl;
         r->phi_rel = hc_.phi_rel; r->dt_reason = hc_.dt_reason; r->phi_passes = hc_.phi_passes;
@@ -326,6 +367,7 @@ public:
 
     void kick(const double* const noise[3], double amp, int passes) override {        // backend.cu:958-978
         probes_fresh_ = false;
+        settle_queued();
         const int S = par_, X2 = par_ ^ 1;
         for (int k = 0; k < 3; k++) {
             const int sx = nx_ + (k == 0), sy = ny_ + (k == 1), sz = nz_ + (k == 2);
@@ -352,6 +394,7 @@ public:
     }
 
     void diagnostics(CavityDiagnostics* d) override {                                  // backend.cu:1096-1129
+        settle_queued();
         OutArgs<T> a = out_args();
         const T lidv = (T)lid_speed_host(hc_.t);
         cell_diag_kernel<T><<<blocks_for(n_cell_), kThreads, 0, stream_>>>(a, lidv);
@@ -389,6 +432,7 @@ public:
 
     void get_field(int field, void* out) override {                                   // backend.cu:1139-1146
         if (field < 0 || field > 6) fail("field must be 0..6");
+        settle_queued();
         if (field == 6) {
             check(cudaMemcpyAsync(out, PHI_[par_], sizeof(double) * n_cell_, cudaMemcpyDeviceToHost, stream_));
         } else {
@@ -401,6 +445,7 @@ public:
     }
     void get_field_f64(int field, double* out) override {
         if (field < 0 || field > 6) fail("field must be 0..6");
+        settle_queued();
         if (field == 6) {
             check(cudaMemcpyAsync(out, PHI_[par_], sizeof(double) * n_cell_, cudaMemcpyDeviceToHost, stream_));
         } else {
@@ -414,6 +459,7 @@ public:
     void set_field(int field, const void* in) override {                              // backend.cu:1147-1155
         probes_fresh_ = false;
         if (field < 0 || field > 6) fail("field must be 0..6");
+        settle_queued();
         if (field == 6) {
             check(cudaMemcpyAsync(PHI_[par_], in, sizeof(double) * n_cell_, cudaMemcpyHostToDevice, stream_));
         } else {
@@ -447,13 +493,17 @@ public:
             step_async(1);
             if (np > 0) {
                 probes_kernel<T><<<1, 32, 0, stream_>>>(out_args(), probe_cells_, np, ring_dev_ + (size_t)ring_n_ * 2 * np);
-                ring_n_++;
+                pending_.back().ring = ring_n_++;
             }
-            if (statistics)
-                statistics_kernel<T><<<blocks_for((long long)nx_ * ny_ + nx_), kThreads, 0, stream_>>>(out_args(), 0.0, ctrl_,
-                                                                                                   stats_, line_);
+            if (statistics) launch_statistics(par_);
+            pending_.back().statistics = statistics != 0;
         }
         check(cudaGetLastError());
+    }
+    // the mid-span statistics of the state of parity `par`, weighted with the dt of the step just taken
+    void launch_statistics(int par) {
+        statistics_kernel<T><<<blocks_for((long long)nx_ * ny_ + nx_), kThreads, 0, stream_>>>(out_args(par), 0.0, ctrl_,
+                                                                                            stats_, line_);
     }
     // waits for the queued steps; copies the probe values of up to max_steps of them (2 n_probes floats each,
     // in order) and returns how many steps they cover
@@ -565,29 +615,35 @@ public:
             std::memcpy(out, tail_probes(), sizeof(float) * 2 * c_.n_probes);
             return;
         }
+        settle_queued();
         probes_kernel<T><<<1, 32, 0, stream_>>>(out_args(), probe_cells_, c_.n_probes, probe_out_);
         check(cudaMemcpyAsync(out, probe_out_, sizeof(float) * 2 * c_.n_probes, cudaMemcpyDeviceToHost, stream_));
         check(cudaStreamSynchronize(stream_));
     }
     void add_statistics(double weight, double* centreline) override {                  // backend.cu:1168-1175
+        settle_queued();
         statistics_kernel<T><<<blocks_for((long long)nx_ * ny_ + nx_), kThreads, 0, stream_>>>(out_args(), weight, nullptr, stats_, line_);
         check(cudaMemcpyAsync(centreline, line_, sizeof(double) * 5 * nx_, cudaMemcpyDeviceToHost, stream_));
         check(cudaStreamSynchronize(stream_));
     }
     void get_statistics(double* sums) override {
+        settle_queued();
         check(cudaMemcpyAsync(sums, stats_, sizeof(double) * 6 * nx_ * ny_, cudaMemcpyDeviceToHost, stream_));
         check(cudaStreamSynchronize(stream_));
     }
     void set_statistics(const double* sums) override {
+        settle_queued();
         check(cudaMemcpyAsync(stats_, sums, sizeof(double) * 6 * nx_ * ny_, cudaMemcpyHostToDevice, stream_));
         check(cudaStreamSynchronize(stream_));
     }
     void midplane(float* out) override {                                               // backend.cu:1178-1184
+        settle_queued();
         midplane_kernel<T><<<blocks_for((long long)nx_ * ny_), kThreads, 0, stream_>>>(out_args(), (T)lid_speed_host(hc_.t), plane_);
         check(cudaMemcpyAsync(out, plane_, sizeof(float) * 4 * nx_ * ny_, cudaMemcpyDeviceToHost, stream_));
         check(cudaStreamSynchronize(stream_));
     }
     void q_volume(int colour_w, float* q, float* colour) override {                    // backend.cu:1185-1194
+        settle_queued();
         const double L_over_U = c_.length / c_.u_lid;
         float* qd = fstage_;
         float* cd = fstage_ + n_cell_;
@@ -631,7 +687,7 @@ public:
                 check(cudaEventRecord(e0, stream_));
                 if (eager_) enqueue_step(par_, timing, true);
                 else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[par_], stream_));
-                pending_.push_back(par_);
+                pending_.push_back({par_});
                 par_ ^= 1;
                 check(cudaEventRecord(e1, stream_));
                 sync(nullptr);
@@ -684,7 +740,7 @@ public:
                 check(cudaEventRecord(e0, stream_));
                 for (int i = 0; i < steps; i++) {
                     check(cudaGraphLaunch(exec_[par_], stream_));
-                    pending_.push_back(par_);
+                    pending_.push_back({par_});
                     par_ ^= 1;
                 }
                 check(cudaEventRecord(e1, stream_));
@@ -932,11 +988,12 @@ private:
         }
     }
 
-    OutArgs<T> out_args() const {
+    OutArgs<T> out_args() const { return out_args(par_); }
+    OutArgs<T> out_args(int par) const {
         OutArgs<T> a;
         a.p = p_;
         a.g = geo_;
-        for (int k = 0; k < 3; k++) { a.u[k] = U_[par_][k]; a.m[k] = M_[par_][k]; }
+        for (int k = 0; k < 3; k++) { a.u[k] = U_[par][k]; a.m[k] = M_[par][k]; }
         a.centre_x = centre_[0];
         a.centre_z = centre_[2];
         a.length_x = (double)(float)ax_[0].length;
@@ -1070,9 +1127,12 @@ private:
         if (between) between();
         if (step_mode) launch_residual(st, praw_, h, use_h, 1);    // the residual of the guess
     }
-    void launch_residual(cudaStream_t st, const double* phi, cudaGraphConditionalHandle h, int use_h, int start = 0) {
+    void launch_residual(cudaStream_t st, const double* phi, cudaGraphConditionalHandle h, int use_h, int start = 0,
+                         int last = 0, int stage = 0) {
         ResidualArgs a;
         a.start = start;
+        a.last = last;
+        a.stage = stage;
         a.p = p_;
         for (int k = 0; k < 3; k++) { a.dw[k] = geo_.dw[k]; a.dinv_sp[k] = geo_.dinv_sp[k]; }
         a.phi = phi;
@@ -1083,12 +1143,23 @@ private:
         a.handle = h;
         a.use_handle = use_h;
         const dim3 grid = column_grid(residual_per_sm_, 2);     // a pair of cells per thread
-        if (!record_launch(kLkResidual, 0, grid, 0, a)) check(launch_pdl(residual_kernel, grid, dim3(kThreads), 0, st, a));
+        if (!record_launch(kLkResidual, 0, grid, 0, a)) check(launch_after(residual_kernel, grid, dim3(kThreads), 0, st, a));
     }
     // one pressure pass (backend.cu:801-814) followed by the residual that decides on the next
     void launch_pass(cudaStream_t st, double* phi, cudaGraphConditionalHandle h, int use_h) {
         launch_transforms(st, phi, h, use_h);
         launch_residual(st, phi, h, use_h);
+    }
+    // the passes of a step's graph without a loop: one, or two on the tensor cores, the last of which may stall the step;
+    // `t0`, `t1`: events around the first pass's transforms
+    void launch_passes(cudaStream_t st, double* phi, int stage, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = nullptr) {
+        if (t0) check(cudaEventRecordWithFlags(t0, st, cudaEventRecordExternal));
+        launch_transforms(st, phi, 0, 0);
+        if (t1) check(cudaEventRecordWithFlags(t1, st, cudaEventRecordExternal));
+        launch_residual(st, phi, 0, 0, 0, !tc_fdm_, stage);
+        if (!tc_fdm_) return;
+        launch_transforms(st, phi, 0, 0);
+        launch_residual(st, phi, 0, 0, 0, 1, stage);
     }
     // the six transforms of a pass (backend.cu:801-814)
     void launch_transforms(cudaStream_t st, double* phi, cudaGraphConditionalHandle h, int use_h) {
@@ -1122,7 +1193,7 @@ private:
         if (!record_launch(kLkFinish, 0, grid, 0, a)) check(launch_pdl(finish_kernel<T>, grid, dim3(kThreads), 0, st, a));
     }
 
-    // A pressure refinement loop inside a stream capture: one pass, then a conditional while-node whose body is
+    // A pressure refinement loop inside a stream capture (loops_): one pass, then a conditional while-node whose body is
     // one pass.  `first_residual` launches the kernels that set the loop condition before them.
     template <class F>
     void captured_loop(F first_residual, double* phi, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = nullptr) {
@@ -1134,8 +1205,8 @@ private:
         cudaGraphConditionalHandle h;
         check(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
         first_residual(h);
-        // the first pass outside the loop: most solves need exactly one, and its kernels skip themselves when the
-        // start decided on none (the first transform clears the loop condition either way)
+        // the first pass outside the loop: its kernels skip themselves when the start decided on none (the first
+        // transform clears the loop condition either way)
         if (t0) check(cudaEventRecordWithFlags(t0, stream_, cudaEventRecordExternal));
         launch_transforms(stream_, phi, h, 1);
         if (t1) check(cudaEventRecordWithFlags(t1, stream_, cudaEventRecordExternal));
@@ -1159,50 +1230,66 @@ private:
     // refinement loops become conditional while-nodes), or eagerly with the loops driven from the host (the
     // launch mode for profilers, which cannot see kernels inside graphs that hold conditional nodes).
     void enqueue_step(int S, bool timing, bool eager) {
-        const int Xs = S ^ 1, Ys = 2;
-        auto mark = [&](cudaEvent_t e) {
-            if (eager) check(cudaEventRecord(e, stream_));
-            else check(cudaEventRecordWithFlags(e, stream_, cudaEventRecordExternal));
-        };
         launch_step_begin(stream_);
-        for (int stage = 0; stage < 3; stage++) {
-            const int in = stage == 0 ? S : stage == 1 ? Xs : Ys;
-            const int out = stage == 1 ? Ys : Xs;
-            const int cur = stage == 1 ? Xs : Ys;          // potential of the previous stage (stages 1, 2)
-            if (timing) mark(kev(kTkSweep, stage)[0]);
-            launch_momentum(stream_, stage, S, in, out);
-            if (timing) mark(kev(kTkSweep, stage)[1]);
-            double* phi = praw_;          // the solve works here; finish writes PHI_[out]
-            // with timing: events around the projection start and around the residual of its guess (one launch where fused)
-            std::function<void()> between;
-            if (timing) mark(kev(kTkStart, stage)[0]);
-            if (timing && !fused_start()) {
-                between = [&, stage] {
-                    mark(kev(kTkStart, stage)[1]);
-                    mark(kev(kTkGuessResidual, stage)[0]);
-                };
-            }
-            if (eager) {
-                launch_start(stream_, M_[out], true, stage, S, cur, 0, 0, between);
-                if (timing) mark(kev(fused_start() ? kTkStart : kTkGuessResidual, stage)[1]);
-                pull_control();
-                for (int pass = 0; hc_.cond && !hc_.error; pass++) {
-                    if (timing && pass == 0) mark(kev(kTkTransforms, stage)[0]);
-                    launch_transforms(stream_, phi, 0, 0);
-                    if (timing && pass == 0) mark(kev(kTkTransforms, stage)[1]);
-                    launch_residual(stream_, phi, 0, 0);
-                    pull_control();
-                }
-            } else {
-                captured_loop([&](cudaGraphConditionalHandle h) {
-                    launch_start(stream_, M_[out], true, stage, S, cur, h, 1, between);
-                    if (timing) mark(kev(fused_start() ? kTkStart : kTkGuessResidual, stage)[1]);
-                }, phi, timing ? kev(kTkTransforms, stage)[0] : nullptr, timing ? kev(kTkTransforms, stage)[1] : nullptr);
-            }
-            if (timing) mark(kev(kTkFinish, stage)[0]);
-            launch_finish(stream_, M_[out], U_[out], PHI_[out], true, stage, stage == 2);
-            if (timing) mark(kev(kTkFinish, stage)[1]);
+        for (int stage = 0; stage < 3; stage++) enqueue_stage(S, stage, timing, eager);
+    }
+    void mark(cudaEvent_t e, bool eager) {
+        if (eager) check(cudaEventRecord(e, stream_));
+        else check(cudaEventRecordWithFlags(e, stream_, cudaEventRecordExternal));
+    }
+    static int stage_out(int S, int stage) { return stage == 1 ? 2 : S ^ 1; }
+    void enqueue_stage(int S, int stage, bool timing, bool eager) {
+        const int Xs = S ^ 1, Ys = 2;
+        const int in = stage == 0 ? S : stage == 1 ? Xs : Ys;
+        const int out = stage_out(S, stage);
+        const int cur = stage == 1 ? Xs : Ys;          // potential of the previous stage (stages 1, 2)
+        if (timing) mark(kev(kTkSweep, stage)[0], eager);
+        launch_momentum(stream_, stage, S, in, out);
+        if (timing) mark(kev(kTkSweep, stage)[1], eager);
+        double* phi = praw_;          // the solve works here; finish writes PHI_[out]
+        // with timing: events around the projection start and around the residual of its guess (one launch where fused)
+        std::function<void()> between;
+        if (timing) mark(kev(kTkStart, stage)[0], eager);
+        if (timing && !fused_start()) {
+            between = [&, stage] {
+                mark(kev(kTkStart, stage)[1], eager);
+                mark(kev(kTkGuessResidual, stage)[0], eager);
+            };
         }
+        cudaEvent_t after_start = timing ? kev(fused_start() ? kTkStart : kTkGuessResidual, stage)[1] : nullptr;
+        cudaEvent_t t0 = timing ? kev(kTkTransforms, stage)[0] : nullptr, t1 = timing ? kev(kTkTransforms, stage)[1] : nullptr;
+        if (eager) {
+            launch_start(stream_, M_[out], true, stage, S, cur, 0, 0, between);
+            if (timing) mark(after_start, true);
+            pull_control();
+            continue_passes(timing, stage);
+        } else if (loops_) {
+            captured_loop([&](cudaGraphConditionalHandle h) {
+                launch_start(stream_, M_[out], true, stage, S, cur, h, 1, between);
+                if (timing) mark(after_start, false);
+            }, phi, t0, t1);
+        } else {
+            launch_start(stream_, M_[out], true, stage, S, cur, 0, 0, between);
+            if (timing) mark(after_start, false);
+            launch_passes(stream_, phi, stage, t0, t1);
+        }
+        finish_stage(S, stage, timing, eager);
+    }
+    // a solve's passes driven from the host, from the control block as last read
+    void continue_passes(bool timing, int stage) {
+        for (int pass = 0; hc_.cond && !hc_.error; pass++) {
+            if (timing && pass == 0) mark(kev(kTkTransforms, stage)[0], true);
+            launch_transforms(stream_, praw_, 0, 0);
+            if (timing && pass == 0) mark(kev(kTkTransforms, stage)[1], true);
+            launch_residual(stream_, praw_, 0, 0);
+            pull_control();
+        }
+    }
+    void finish_stage(int S, int stage, bool timing, bool eager) {
+        const int out = stage_out(S, stage);
+        if (timing) mark(kev(kTkFinish, stage)[0], eager);
+        launch_finish(stream_, M_[out], U_[out], PHI_[out], true, stage, stage == 2);
+        if (timing) mark(kev(kTkFinish, stage)[1], eager);
     }
 
     void build_graphs() {
@@ -1318,7 +1405,14 @@ private:
         const long long zc = (nz_ + chunks - 1) / chunks;
         return (unsigned int)((nz_ + zc - 1) / zc);
     }
-    std::vector<int> pending_;
+    // a queued step: its state parity, its slot in the ring of probe values (-1: none), whether statistics follow it
+    struct Pending {
+        int par, ring = -1;
+        bool statistics = false;
+    };
+    std::vector<Pending> pending_;
+    bool batch_pending_ = false;        // queued by a batch
+    bool loops_ = false;                // step graphs with conditional refinement loops (after a stalled solve)
     long long steps_before_ = 0;
     // fields: three buffer sets of velocity, impulse and potential (state, stage outputs)
     T* U_[3][3];
@@ -1444,6 +1538,7 @@ public:
         if (f.tc_fdm_) check(tc_transform_prepare_batched());
         if (f.tc_fdm_) check(tc_pair_prepare());
         check(pair_prepare());
+        for (const S_* s : m_) loops_ = loops_ || (s && s->loops_);
         for (int S = 0; S < 2; S++) build(S);
         proto_ = nullptr;        // members may leave and be destroyed from now on
     }
@@ -1463,6 +1558,13 @@ public:
     int size() const override { return (int)m_.size(); }
 
     void step_async(int count) override {
+        if (!queued_ && !loops_) {       // a member's solve stalled (Solver::settle): graphs with refinement loops from now on
+            for (S_* s : m_)
+                if (s && s->loops_) {
+                    rebuild_with_loops(s);
+                    break;
+                }
+        }
         for (int i = 0; i < count; i++) launch_step(exec_);
     }
     // Per-step device time (ms, summed over the three stages) of the batch's parts: the sweeps, the projection
@@ -1509,7 +1611,8 @@ private:
             for (S_* s : m_) {
                 if (!s) continue;
                 if (s->pending_.empty()) s->steps_before_ = s->hc_.steps;
-                s->pending_.push_back(s->par_);
+                s->pending_.push_back({s->par_});
+                s->batch_pending_ = true;
                 s->par_ ^= 1;
                 s->tail_queued_ = false;          // a batch step has no per-cavity tail: sync reads the control block
                 s->probes_fresh_ = false;
@@ -1631,13 +1734,19 @@ private:
         const int in = stage == 0 ? Sm : stage == 1 ? Xs : Ys;
         const int out = stage == 1 ? Ys : Xs;
         const int cur = stage == 1 ? Xs : Ys;
-        const cudaGraphConditionalHandle h = handles_[S][stage];
+        const cudaGraphConditionalHandle h = loops_ ? handles_[S][stage] : 0;
         cudaStream_t st = part == 3 ? body_stream_ : stream_;
         switch (part) {
         case 0: s.launch_momentum(st, stage, Sm, in, out); break;
-        case 1: s.launch_start(st, s.M_[out], true, stage, Sm, cur, h, 2); break;
+        case 1: s.launch_start(st, s.M_[out], true, stage, Sm, cur, h, loops_ ? 2 : 0); break;
         case 2:
-        case 3: s.launch_pass(st, s.praw_, h, 2); break;
+            if (!loops_) {
+                s.launch_passes(st, s.praw_, stage);
+                break;
+            }
+        case 3:
+            if (loops_) s.launch_pass(st, s.praw_, h, 2);
+            break;
         case 4: s.launch_finish(st, s.M_[out], s.U_[out], s.PHI_[out], true, stage, stage == 2); break;
         }
     }
@@ -1729,7 +1838,7 @@ private:
                 check(launch_pdl(projection_start_batched<T>, g, dim3(kThreads), 0, st, (const StartArgs<T>*)d, items, live));
             break;
         case kLkResidual:
-            check(launch_pdl(residual_batched, g, dim3(kThreads), 0, st, (const ResidualArgs*)d, items, live));
+            check(launch_after(residual_batched, g, dim3(kThreads), 0, st, (const ResidualArgs*)d, items, live));
             break;
         case kLkFinish:
             check(launch_pdl(finish_batched<T>, g, dim3(kThreads), 0, st, (const FinishArgs<T>*)d, items, live));
@@ -1770,7 +1879,7 @@ private:
             const cudaGraphNode_t* deps = nullptr;
             size_t ndeps = 0;
             cudaStreamCaptureStatus status;
-            if (launch) {
+            if (launch && loops_) {
                 check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &g, &deps, &ndeps));
                 check(cudaGraphConditionalHandleCreate(&handles_[S][stage], g, 0, cudaGraphCondAssignDefault));
             }
@@ -1781,7 +1890,9 @@ private:
             mark(stage, 2, 0);
             emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 2); }, host, L, launch);
             mark(stage, 2, 1);
-            if (launch) {
+            if (!loops_) {
+                // the passes are all in the chain
+            } else if (launch) {
                 check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &g, &deps, &ndeps));
                 cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
                 cp.type = cudaGraphNodeTypeConditional;
@@ -1802,6 +1913,21 @@ private:
             emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 4); }, host, L, launch);
             mark(stage, 3, 1);
         }
+    }
+    // the plain graphs again, with refinement loops; empty slots record `proto`
+    void rebuild_with_loops(S_* proto) {
+        loops_ = true;
+        proto_ = proto;
+        for (int S = 0; S < 2; S++) {
+            check(cudaGraphExecDestroy(exec_[S]));
+            check(cudaGraphDestroy(graph_[S]));
+            check(cudaFree(dargs_[S]));
+            exec_[S] = nullptr;
+            graph_[S] = nullptr;
+            dargs_[S] = nullptr;
+            build(S);
+        }
+        proto_ = nullptr;
     }
     // the step graph of batch parity S; with `timing` the instrumented twin (part_times), built from the current
     // members with its own argument buffer and refinement-loop handles (the plain graph's are kept)
@@ -1862,6 +1988,7 @@ private:
     Layout layout_[2];
     bool mixed_sizes_ = false;
     int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 64 cells)
+    bool loops_ = false;        // conditional refinement loops in the graphs
     bool fused_start_ = false;  // projection starts with their guesses' residuals in one launch
     int tc_pairs_ = 0;          // tensor-core passes as paired launches (g_batch_tc_pairs)
     int dgemm_tile_ = 0;

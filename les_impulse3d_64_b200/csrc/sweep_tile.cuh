@@ -172,7 +172,6 @@ template <class T, class G> __device__ __forceinline__ TileArrays<T> tile_arrays
 template <class T, class G>
 __device__ bool tile_prologue(const MomentumArgs<T>& a, const Blk& blk, const TileArrays<T>& t, StageConst& sc, T& dt) {
     constexpr int TY = G::TYc, TZ = G::TZc, NT = G::THREADS;
-    pdl_launch_dependents();
     pdl_wait();
     constexpr int TX = G::TX;
     constexpr int UW = G::UW, UH = G::UH, VW = G::VW, VH = G::VH, WW = G::WW, WH = G::WH, MW = G::MW, MH = G::MH;
@@ -236,6 +235,7 @@ __device__ bool tile_prologue(const MomentumArgs<T>& a, const Blk& blk, const Ti
         __syncthreads();
     }
 
+    pdl_launch_dependents();
     // ---- K = u.m per cell (x0-1+ix, y0-1+iy, z0-1+iz)
     constexpr int KW = TX + 1, KRPS = NT / KW;
     for (int e = threadIdx.x % KW + KW * (threadIdx.x / KW); threadIdx.x < KRPS * KW && e < G::NK; e += KRPS * KW) {
