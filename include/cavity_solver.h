@@ -105,7 +105,7 @@ int cavity_time_steps(CavitySolver* s, int warmup, int steps, int flush_l2, floa
  * sweep (the tile kernel, in FP32 also its packed two-cells-per-thread form, or the z-march with 1/2, 1, 2 or 4
  * times its device-filling z-chunk count; only the
  * kernel CAVITY_SWEEP names, when set), then the FP64 transforms (six launches of 64 x 64 or 32 x 32 tiles, one
- * cooperative launch of 32 x 32 tiles, or, where no axis exceeds 64 cells, three launches of two chained
+ * cooperative launch of 32 x 32 tiles, or, where no axis exceeds 128 cells, three launches of two chained
  * transforms each).  The choice is cached per grid size, stretching and precision form
  * for the process, and in the file named by CAVITY_TUNE_FILE when that is set; cavities created later with the
  * same key start with it.  The transform choices and the chunk counts give bit-identical steps; the two sweep

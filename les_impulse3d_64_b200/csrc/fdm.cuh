@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(WARPS_M * WARPS_N * 32) dgemm_mma_batched(cons
 // Every dot product runs over k in the same order, four at a time from a zero accumulator, as in
 // dgemm_mma_body, and the values between the transforms are the same doubles, so each transform's result is
 // bit for bit the six-launch pass's.  Shared-memory operands are zero outside the matrices up to the next
-// multiple of 8 (rows) or 4 (k), as the six-launch pass's staged panels are.
-constexpr int kPairMax = 64;                 // the largest axis a paired pass takes
+// multiple of 8 (rows) or 4 (k), as the six-launch pass's staged panels are.  A launch with a longer axis, to 128 cells,
+// is pair_wide_kernel's.
+constexpr int kPairMax = 64;                 // the largest axis these three take
 constexpr int kPairPitch = kPairMax + 4;     // row pitch of a 64-wide operand: 8 banks mod 32
 constexpr int kPairThreads = 256;
 
@@ -471,6 +472,219 @@ template <int W> struct PairYxSmem {
     static constexpr size_t bytes = sizeof(double) * (2 * kPairMax * kPairPitch + 2 * W * kPairPitch);
 };
 
+// The same three launches for axes of up to kWideMax cells, whose planes and bases no longer fit in shared memory
+// together: a CTA's operands stream through a ring of K panels (cp.async, kWideStages - 1 ahead), and only the
+// intermediate of the chained transforms stays.  8 warps own 16 x 32 values each: 128 rows x 32 columns (xy, z), 32 rows
+// x 128 columns (yx); fragments outside the matrices are skipped.  The dot products run in the same order as
+// dgemm_mma_body's, so the pass is bit for bit the six-launch one.
+// What bounds the six launches there is the fixed part of each, about 8 us of launch, first loads, a last uneven wave
+// and stores beside 5 to 6 us of products at 96^3; three launches have it half as often and keep every second
+// intermediate out of memory.  Measured, us of a step's first passes, six launches and three: 96^3 303 and 237 (the step
+// 588 and 519), 100 x 100 x 75 349 and 307 (817 and 775), 64 x 64 x 128 (xy and yx by the kernels above) 167 and 140
+// (374 and 346), 128^3 673 and 571.  Two or four panels of 16 in the ring of the six launches' tile GEMM, or skipping
+// its outside fragments, gave nothing (349 to 372 at 100 x 100 x 75).
+constexpr int kWideMax = 128, kWideW = 32, kWideKC = 16, kWideStages = 3;
+struct WideSmem {
+    static constexpr int LDA = kWideKC + 4;                      // pitch of an A panel (rows x K)
+    static constexpr int PN = kWideW + 4, PX = kWideMax + 4;     // pitches of 32- and 128-column operands
+    static constexpr int STAGE = kWideMax * LDA + kWideKC * PN > kWideW * LDA + kWideKC * PX
+                                     ? kWideMax * LDA + kWideKC * PN : kWideW * LDA + kWideKC * PX;
+    static constexpr int MID = kWideMax * PN > kWideW * PX ? kWideMax * PN : kWideW * PX;
+    static constexpr size_t bytes = sizeof(double) * (kWideStages * STAGE + MID);
+};
+// rows [0, R) x [0, C) of a panel at dst (pitch P) from src (pitch ld) where (row, col) exist, else zero; C is even
+template <int R, int C, int P>
+__device__ __forceinline__ void wide_stage(double* dst, const double* src, long long ld, int rows, int cols) {
+    const bool two = ld % 2 == 0 && ((unsigned long long)src & 15) == 0;
+    for (int e = threadIdx.x; e < R * C / 2; e += kPairThreads) {
+        const int r = e / (C / 2), c = 2 * (e % (C / 2));
+        const int n = r < rows ? min(2, max(0, cols - c)) : 0;
+        const double* q = src + r * ld + c;
+        if (two) {
+            cp_async16z(dst + r * P + c, n ? q : src, 8 * n);
+        } else {
+            cp_async8(dst + r * P + c, n > 0 ? q : src, n > 0 ? 8 : 0);
+            cp_async8(dst + r * P + c + 1, n > 1 ? q + 1 : src, n > 1 ? 8 : 0);
+        }
+    }
+}
+// One transform of a CTA: acc = A (M x K) B (K x N) on this warp's 16 rows from mw and 32 columns from nw.  A_STREAM,
+// B_STREAM: the operand comes panel by panel from global memory (MT rows of A, NT columns of B in the tile), else it
+// is resident in shared memory with pitch LDM.
+template <int MT, int NT, int LDM, bool A_STREAM, bool B_STREAM>
+__device__ __forceinline__ void wide_transform(double (&acc)[2][4][2], double* ring, const double* mid, const double* A,
+                                               long long lda, int M, const double* B, long long ldb, int N, int K, int mw,
+                                               int nw) {
+    constexpr int LDA = WideSmem::LDA, PB = NT + 4;
+    const int lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
+    const int fm = min(2, max(0, (M - mw + 7) / 8)), fn = min(4, max(0, (N - nw + 7) / 8));
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    const int panels = (K + kWideKC - 1) / kWideKC;
+    auto issue = [&](int p) {
+        double* s = ring + (p % kWideStages) * WideSmem::STAGE;
+        const int k0 = p * kWideKC;
+        if (A_STREAM) wide_stage<MT, kWideKC, LDA>(s, A + k0, lda, M, K - k0);
+        if (B_STREAM) wide_stage<kWideKC, NT, PB>(s + MT * LDA, B + k0 * ldb, ldb, K - k0, N);
+    };
+#pragma unroll
+    for (int p = 0; p < kWideStages - 1; p++) {
+        if (p < panels) issue(p);
+        cp_async_commit();
+    }
+    for (int p = 0; p < panels; p++) {
+        cp_async_wait<kWideStages - 2>();
+        __syncthreads();                                    // panel p has landed, panel p - 1 is no longer read
+        if (p + kWideStages - 1 < panels) issue(p + kWideStages - 1);
+        cp_async_commit();
+        const double* s = ring + (p % kWideStages) * WideSmem::STAGE;
+        const double* a = A_STREAM ? s + (mw + fr) * LDA + fc : mid + (mw + fr) * LDM + p * kWideKC + fc;
+        const double* b = B_STREAM ? s + MT * LDA + fc * PB + nw + fr : mid + (p * kWideKC + fc) * LDM + nw + fr;
+        constexpr int sa = A_STREAM ? LDA : LDM, sb = B_STREAM ? PB : LDM;
+        const int kend = min(kWideKC, K - p * kWideKC);
+        if (fm == 0 || fn == 0) continue;
+        for (int kk = 0; kk < kend; kk += 4) {
+            double af[2], bf[4];
+#pragma unroll
+            for (int i = 0; i < 2; i++) af[i] = a[i * 8 * sa + kk];
+#pragma unroll
+            for (int j = 0; j < 4; j++) bf[j] = b[kk * sb + j * 8];
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (i < fm && j < fn) dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        }
+    }
+}
+
+template <int PHASE>
+__device__ void pair_wide_body(const FdmPairArgs& a, const Blk& blk, bool first) {
+    pair_begin(a, first, PHASE == 0);
+    extern __shared__ __align__(16) double pair_smem[];
+    double* ring = pair_smem;
+    double* mid = ring + kWideStages * WideSmem::STAGE;
+    constexpr int PN = WideSmem::PN, PX = WideSmem::PX;
+    if (!pair_live(a)) return;
+    const int nx = a.nx, ny = a.ny, nz = a.nz, plane = nx * ny;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
+    double acc[2][4][2];
+    // rows of the intermediate that the second transform's last k step reads beyond its K are zero: a streamed operand
+    // is zero there already, and 0 times a stale value could be NaN
+    for (int e = threadIdx.x; e < WideSmem::MID; e += kPairThreads) mid[e] = 0.0;
+    __syncthreads();
+    if (PHASE != 2) {
+        const bool z = PHASE == 1;
+        const int mw = warp * 16, col0 = blk.x * kWideW, M = z ? nz : ny;
+        const int N = min(kWideW, (z ? plane : nx) - col0);
+        const double* r = PHASE == 0 ? (a.r_alt && a.c->use_rhs ? a.r_alt : a.r) + (long long)blk.y * plane : nullptr;
+        const double* t_in = a.t + col0;
+        double il[2][4][2];                                     // 1/lambda of this thread's values, loaded ahead
+        if (z) {
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int row = mw + i * 8 + fr, col = j * 8 + 2 * fc + h;
+                        il[i][j][h] = row < M && col < N ? __ldg(a.inv_lambda + (long long)row * plane + col0 + col) : 0.0;
+                    }
+        }
+        if (z) wide_transform<kWideMax, kWideW, 0, true, true>(acc, ring, nullptr, a.st[Z], nz, nz, t_in, plane, N, nz, mw, 0);
+        else wide_transform<kWideMax, kWideW, 0, true, true>(acc, ring, nullptr, r, nx, ny, a.s[X] + col0, nx, N, nx, mw, 0);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int row = mw + i * 8 + fr, col = j * 8 + 2 * fc + h;
+                    if (row >= M || col >= N) continue;
+                    const double v = acc[i][j][h];
+                    mid[row * PN + col] = z ? v * il[i][j][h] : v;
+                }
+        __syncthreads();
+        const double* basis = z ? a.s[Z] : a.st[Y];
+        wide_transform<kWideMax, kWideW, PN, true, false>(acc, ring, mid, basis, M, M, nullptr, 0, N, M, mw, 0);
+        pdl_launch_dependents();
+        double* t = z ? a.t + col0 : a.t + (long long)blk.y * plane + col0;
+        const long long ld = z ? plane : nx;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int row = mw + i * 8 + fr;
+            if (row >= M) continue;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int col = j * 8 + 2 * fc + h;
+                    if (col < N) t[row * ld + col] = acc[i][j][h];
+                }
+        }
+    } else {
+        const int mw = (warp >> 2) * 16, nw = (warp & 3) * 32, y0 = blk.x * kWideW, M = min(kWideW, ny - y0);
+        const long long at = (long long)blk.y * plane;
+        wide_transform<kWideW, kWideMax, 0, true, true>(acc, ring, nullptr, a.s[Y] + (long long)y0 * ny, ny, M, a.t + at, nx,
+                                                        nx, ny, mw, nw);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int row = mw + i * 8 + fr, col = nw + j * 8 + 2 * fc + h;
+                    if (row < M && col < nx) mid[row * PX + col] = acc[i][j][h];
+                }
+        // the potential this thread updates, loaded under the second transform
+        const int reset = a.c->reset_phi;
+        double* phi = a.phi + at + (long long)y0 * nx;
+        double old[2][4][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int row = mw + i * 8 + fr, col = nw + j * 8 + 2 * fc + h;
+                    old[i][j][h] = row < M && col < nx && !reset ? phi[row * nx + col] : 0.0;
+                }
+        __syncthreads();
+        wide_transform<kWideW, kWideMax, PX, false, true>(acc, ring, mid, nullptr, 0, M, a.st[X], nx, nx, nx, mw, nw);
+        pdl_launch_dependents();
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int row = mw + i * 8 + fr;
+            if (row >= M) continue;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int col = nw + j * 8 + 2 * fc + h;
+                    if (col < nx) phi[row * nx + col] = old[i][j][h] + acc[i][j][h];
+                }
+        }
+    }
+}
+template <int PHASE> __global__ void __launch_bounds__(kPairThreads, 2) pair_wide_kernel(FdmPairArgs a) {
+    pair_wide_body<PHASE>(a, real_blk(), first_block());
+}
+template <int PHASE>
+__global__ void __launch_bounds__(kPairThreads, 2) pair_wide_batched(const FdmPairArgs* args, const BatchItem* items,
+                                                                    const int* live) {
+    __shared__ FdmPairArgs a;
+    int cav;
+    const Blk k = item_blk(items, live, cav);
+    if (cav < 0) {
+        if (PHASE == 0) dead_slot_clear(args, items);
+        return;
+    }
+    load_args(a, args + cav);
+    pair_wide_body<PHASE>(a, k, first_block());
+}
+
 enum PairPhase : int { kPairXy = 0, kPairZ = 1, kPairYx = 2 };
 
 template <int W> __global__ void __launch_bounds__(kPairThreads, 2) pair_xy_kernel(FdmPairArgs a) {
@@ -498,6 +712,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_batched(const FdmPairArg
     else if (PHASE == kPairZ) pair_z_body<W>(a, k, first_block());
     else pair_yx_body<W>(a, k, first_block());
 }
+constexpr int kPairWideVariant = 1;          // in the width field of a recorded launch: the streamed kernel
 inline size_t pair_smem_bytes(int phase, int w) {
     if (w == 16) return phase == kPairYx ? PairYxSmem<16>::bytes : PairSmem<16>::bytes;
     return phase == kPairYx ? PairYxSmem<32>::bytes : PairSmem<32>::bytes;
@@ -509,7 +724,12 @@ inline dim3 pair_grid(int phase, int w, int nx, int ny, int nz, int per = 1) {
     return dim3((ny + w - 1) / w, (nz + per - 1) / per);
 }
 inline bool pair_pass_fits(int nx, int ny, int nz) {
-    return nx <= kPairMax && ny <= kPairMax && nz <= kPairMax;
+    return nx <= kWideMax && ny <= kWideMax && nz <= kWideMax;
+}
+// whether a phase's axes need the streamed kernel (a batch runs one kernel for all its members: g_batch_wide)
+inline bool pair_wide(int phase, int nx, int ny, int nz) {
+    if (g_launch_record) return (g_batch_wide >> phase) & 1;
+    return phase == kPairZ ? nz > kPairMax : nx > kPairMax || ny > kPairMax;
 }
 inline int current_sm_count() {
     int dev = 0, sms = 148;
@@ -575,8 +795,13 @@ template <int W> inline cudaError_t pair_prepare_w() {
 // once per process, before any capture: the dynamic shared memory of the paired kernels
 inline cudaError_t pair_prepare() {
     static const cudaError_t e = [] {
-        const cudaError_t r = pair_prepare_w<32>();
-        return r == cudaSuccess ? pair_prepare_w<16>() : r;
+        cudaError_t r = pair_prepare_w<32>();
+        if (r == cudaSuccess) r = pair_prepare_w<16>();
+        for (const void* f : {(const void*)pair_wide_kernel<kPairXy>, (const void*)pair_wide_kernel<kPairZ>,
+                              (const void*)pair_wide_kernel<kPairYx>, (const void*)pair_wide_batched<kPairXy>,
+                              (const void*)pair_wide_batched<kPairZ>, (const void*)pair_wide_batched<kPairYx>})
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideSmem::bytes);
+        return r;
     }();
     return e;
 }
@@ -586,6 +811,15 @@ inline void launch_pair_w(int phase, dim3 grid, cudaStream_t st, const FdmPairAr
     if (phase == kPairXy) launch_pdl(pair_xy_kernel<W>, grid, dim3(kPairThreads), smem, st, a);
     else if (phase == kPairZ) launch_pdl(pair_z_kernel<W>, grid, dim3(kPairThreads), smem, st, a);
     else launch_pdl(pair_yx_kernel<W>, grid, dim3(kPairThreads), smem, st, a);
+}
+// A launch with fewer CTAs than SMs starts when its predecessor is done: started under its tail, its CTAs go two to an SM
+// wherever that tail has left one, while other SMs stay without (64 x 64 x 128, whose z phase has 128 CTAs: step 381 us,
+// so 346); 96^3 and 100 x 100 x 75, with 288 and 313, are 0.3% faster started early.
+inline void launch_wide(void (*kernel)(FdmPairArgs), dim3 grid, cudaStream_t st, const FdmPairArgs& a) {
+    static const int sms = current_sm_count();
+    const dim3 block(kPairThreads);
+    if ((long long)grid.x * grid.y < sms) launch_after(kernel, grid, block, WideSmem::bytes, st, a);
+    else launch_pdl(kernel, grid, block, WideSmem::bytes, st, a);
 }
 inline void launch_fdm_pass_pairs(cudaStream_t st, const FdmOperands& op, const double* r, const double* r_alt,
                                   double* phi, double* t, const Control* c, cudaGraphConditionalHandle h, bool clear) {
@@ -597,6 +831,15 @@ inline void launch_fdm_pass_pairs(cudaStream_t st, const FdmOperands& op, const 
     a.r = r; a.r_alt = r_alt; a.t = t; a.phi = phi; a.c = c; a.handle = h;
     const int w = pair_width(op.nx, op.nz);
     for (int ph = 0; ph < 3; ph++) {
+        if (pair_wide(ph, op.nx, op.ny, op.nz)) {
+            a.per = 1;
+            const dim3 grid = pair_grid(ph, kWideW, op.nx, op.ny, op.nz, 1);
+            if (record_launch(kLkPair, ph | (kPairWideVariant << 4), grid, WideSmem::bytes, a)) continue;
+            if (ph == kPairXy) launch_wide(pair_wide_kernel<kPairXy>, grid, st, a);
+            else if (ph == kPairZ) launch_wide(pair_wide_kernel<kPairZ>, grid, st, a);
+            else launch_wide(pair_wide_kernel<kPairYx>, grid, st, a);
+            continue;
+        }
         a.per = pair_per(ph, w, op.nx, op.ny, op.nz);
         const dim3 grid = pair_grid(ph, w, op.nx, op.ny, op.nz, a.per);
         if (record_launch(kLkPair, ph | (w << 4), grid, pair_smem_bytes(ph, w), a)) continue;
@@ -615,6 +858,14 @@ inline void launch_pair_batched_w(int phase, dim3 grid, const BatchItem* items, 
 }
 inline void launch_pair_batched(int variant, dim3 grid, const BatchItem* items, const int* live, const FdmPairArgs* d,
                                 cudaStream_t st) {
+    if ((variant >> 4) == kPairWideVariant) {
+        const int ph = variant & 15;
+        const dim3 block(kPairThreads);
+        if (ph == kPairXy) launch_pdl(pair_wide_batched<kPairXy>, grid, block, WideSmem::bytes, st, d, items, live);
+        else if (ph == kPairZ) launch_pdl(pair_wide_batched<kPairZ>, grid, block, WideSmem::bytes, st, d, items, live);
+        else launch_pdl(pair_wide_batched<kPairYx>, grid, block, WideSmem::bytes, st, d, items, live);
+        return;
+    }
     if ((variant >> 4) == 16) launch_pair_batched_w<16>(variant & 15, grid, items, live, d, st);
     else launch_pair_batched_w<32>(variant & 15, grid, items, live, d, st);
 }
@@ -771,7 +1022,7 @@ inline void launch_fdm_pass_fused(cudaStream_t st, const FdmOperands& op, const 
 //   kPassOneLaunch:  one cooperative launch with grid barriers (single cavities only).  It is not a default: inside
 //                    the step graph it measured slower than six launches (C2 step 0.383 against 0.368 ms), the
 //                    graph's programmatic launches already hiding most of the gaps that the grid barriers replace;
-//   kPassPairs:      three launches of two chained transforms each, when no axis has more than 64 cells: the
+//   kPassPairs:      three launches of two chained transforms each, when no axis has more than 128 cells: the
 //                    default there.
 // A batch's launches follow the batch's choice (g_batch_pairs), the same for every member.
 enum PassForm : int { kPassSix = 0, kPassOneLaunch = 1, kPassPairs = 2 };

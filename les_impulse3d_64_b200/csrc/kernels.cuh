@@ -45,6 +45,8 @@ inline thread_local int g_launch_batch = 1;
 inline thread_local int g_dgemm_tile = 0;
 // a batch's FP64 passes as three paired launches (1) or six (0); -1 outside a batch
 inline thread_local int g_batch_pairs = -1;
+// the phases (bits) of a batch's paired passes that run the streamed kernel for axes beyond 64 cells (fdm.cuh)
+inline thread_local int g_batch_wide = 0;
 // a batch's tensor-core passes as three paired launches (1: members of one size, 2: of several) or six (0); -1
 // outside a batch
 inline thread_local int g_batch_tc_pairs = -1;

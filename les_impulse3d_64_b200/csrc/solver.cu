@@ -717,7 +717,7 @@ public:
     // 2 and 4 times its device-filling z-chunk count;
     // only the chosen kernel when CAVITY_SWEEP names one), then, with the fastest sweep, the FP64 transforms where
     // they run (64 x 64 tiles, 32 x 32 tiles, 32 x 32 tiles in one cooperative launch, and three paired launches
-    // where no axis exceeds 64 cells).
+    // where no axis exceeds 128 cells).
     void autotune(int steps, int* chunks_out, int* dgemm_out, int* fused_out, float* ms_out) override {
         if (!pending_.empty()) fail("autotune: steps are queued; sync first");
         steps = std::max(steps, 2);
@@ -1500,12 +1500,14 @@ public:
         // have two 64 x 64 tiles per SM in the largest transform
         if (mixed_sizes_) dgemm_tile_ = tiles64 >= 2 * f.sms_ ? 64 : 32;
         // FP64 passes as paired launches when every member's axes allow them (and CAVITY_FDM_FUSED names no
-        // other form)
+        // other form), a phase by the streamed kernel when any member needs it
         {
             bool fits = true;
             for (const S_* s : m_) fits = fits && pair_pass_fits(s->nx_, s->ny_, s->nz_);
             const int e = pass_form_from_env();
             pairs_ = fits && (e < 0 || e == kPassPairs) ? 1 : 0;
+            for (const S_* s : m_)
+                for (int ph = 0; ph < 3; ph++) wide_ |= pair_wide(ph, s->nx_, s->ny_, s->nz_) << ph;
             bool tc_fits = true;
             for (const S_* s : m_) tc_fits = tc_fits && tc_pair_fits(s->nx_, s->ny_, s->nz_);
             tc_pairs_ = !tc_fits ? 0 : mixed_sizes_ ? 2 : 1;
@@ -1665,7 +1667,7 @@ public:
             for (int S = 0; S < 2; S++) {
                 std::vector<LaunchRecord> rec;
                 {
-                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_);
+                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_);
                     record_member(*s, S ^ d_[slot], S);
                 }
                 const Layout& L = layout_[S];
@@ -1690,13 +1692,15 @@ public:
 
 private:
     struct RecordGuard {
-        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs, bool fused_start) {
+        RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs, bool fused_start,
+                    int wide) {
             g_launch_record = r;
             g_launch_batch = batch;
             g_dgemm_tile = dgemm_tile;
             g_batch_pairs = pairs;
             g_batch_tc_pairs = tc_pairs;
             g_batch_fused_start = fused_start;
+            g_batch_wide = wide;
         }
         ~RecordGuard() {
             g_launch_record = nullptr;
@@ -1705,6 +1709,7 @@ private:
             g_batch_pairs = -1;
             g_batch_tc_pairs = -1;
             g_batch_fused_start = false;
+            g_batch_wide = 0;
         }
     };
     static size_t align256(size_t n) { return (n + 255) / 256 * 256; }
@@ -1763,7 +1768,7 @@ private:
         const size_t B = m_.size();
         std::vector<std::vector<LaunchRecord>> recs(B);
         for (size_t b = 0; b < B; b++) {
-            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_);
+            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_);
             if (m_[b]) fn(*m_[b], (int)b);
             else fn(*proto_, 0);
         }
@@ -1987,7 +1992,8 @@ private:
     std::vector<unsigned char> host_[2];      // host copies of the argument buffers
     Layout layout_[2];
     bool mixed_sizes_ = false;
-    int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 64 cells)
+    int wide_ = 0;              // the phases of the paired pass that run the streamed kernel (g_batch_wide)
+    int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 128 cells)
     bool loops_ = false;        // conditional refinement loops in the graphs
     bool fused_start_ = false;  // projection starts with their guesses' residuals in one launch
     int tc_pairs_ = 0;          // tensor-core passes as paired launches (g_batch_tc_pairs)
