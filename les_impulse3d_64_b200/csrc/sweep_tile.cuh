@@ -9,7 +9,7 @@
 //     boxes' cells);
 //   - the slices of the per-axis coefficient tables the tile uses.
 // No thread waits on a global load while staging: every element is a cp.async, all in flight together.
-// Staged values outside the box are clamped copies; every stencil term that reaches them has weight zero.
+// Staged values outside the box are clamped copies (y, z) or zeros (x); every stencil term that reaches them has weight zero.
 // K = u.m (backend.cu:218-222) is computed once per cell.  Each face then adds its eight edge terms
 // (vorticity times interpolated velocity: backend.cu:141-215), evaluated from shared memory, in the
 // reference's order: narrow then wide stencil, first then second tangential axis (backend.cu:232-238,
@@ -71,6 +71,14 @@ __device__ __forceinline__ void cp_async_elem(void* smem_dst, const void* src) {
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src));
 }
 
+// the same copying `bytes` bytes, all or none, and zeros for the rest
+template <int BYTES>
+__device__ __forceinline__ void cp_async_or_zero(void* smem_dst, const void* src, int bytes) {
+    const unsigned int dst = (unsigned int)__cvta_generic_to_shared(smem_dst);
+    if (BYTES == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+
 // Global offsets of the rows (y, z) of a W x H x D box of a face array with extents (ex, ey, ez) whose corner is
 // (., ys, zs), clamped into the array; rows are numbered iy + H * iz.
 template <int H, int D>
@@ -79,9 +87,12 @@ __device__ __forceinline__ int box_row_base(int row, int ys, int zs, int ex, int
     return ex * (clampi(ys + iy, 0, ey - 1) + ey * clampi(zs + iz, 0, ez - 1));
 }
 
-// Stage a W x H x D box of a face array whose x-extent is ex and corner x is xs, coordinates clamped into the
-// array, from the row offsets `rowbase` (box_row_base), rows P apart in `dst`.  Each thread keeps one column (its
-// x offset and clamp) and steps through the rows NT / W at a time.
+// Stage a W x H x D box of a face array whose x-extent is ex and corner x is xs, from the row offsets `rowbase`
+// (box_row_base: y and z clamped into the array), rows P apart in `dst`; columns outside the array are zero.  Each thread
+// keeps one column (its x offset) and steps through the rows NT / W at a time.  Lanes that all copied the same clamped
+// element would take turns: us per step's sweeps with clamped columns and with zeros 322 and 266 (100 x 100 x 75, FP64;
+// the last tile has 4 of 32 columns), 67 and 51 (50 x 50 x 37, FP64), 542 and 468 (164 x 164 x 93, FP32), 99 and 98 (64^3,
+// FP64, where only the rim is outside).  Zeros stored by a branch of their own took 278 and 101 at the first and the last.
 template <class T, int W, int P, int H, int D, int NT>
 __device__ __forceinline__ void stage_box(T* dst, const int* rowbase, const T* __restrict__ m, int xs, int ex) {
     constexpr int RPS = NT / W, ROWS = H * D;
@@ -89,7 +100,8 @@ __device__ __forceinline__ void stage_box(T* dst, const int* rowbase, const T* _
     if (t >= RPS * W) return;
     const int ix = t % W;
     const int gx = clampi(xs + ix, 0, ex - 1);
-    for (int row = t / W; row < ROWS; row += RPS) cp_async_elem<sizeof(T)>(dst + row * P + ix, m + rowbase[row] + gx);
+    const int bytes = gx == xs + ix ? sizeof(T) : 0;
+    for (int row = t / W; row < ROWS; row += RPS) cp_async_or_zero<sizeof(T)>(dst + row * P + ix, m + rowbase[row] + gx, bytes);
 }
 // Stage 0's gauge-reset blend of a staged impulse box (MC columns, row pitch MW): m <- r m + (1-r) u, with u at
 // the same face from the velocity box (plane / row strides VP, VW; `uoff` its offset of the impulse box's corner)
