@@ -29,7 +29,7 @@ namespace cavity {
 // launch (kind, template variant, grid, dynamic shared memory and argument record) to it instead of launching:
 // a batch of cavities collects every member's arguments for the same launch sequence this way and issues one
 // batched launch per entry.
-enum SweepKind : int { kSweepFace = 0, kSweepTile = 1, kSweepMarch = 2, kSweepPair = 3 };
+enum SweepKind : int { kSweepFace = 0, kSweepTile = 1, kSweepMarch = 2, kSweepPair = 3, kSweepColumn = 4 };
 enum LaunchKind : int { kLkStepBegin = 0, kLkSweep, kLkStart, kLkResidual, kLkFinish, kLkDgemm64, kLkDgemm32, kLkTc,
                         kLkPair, kLkTcPair };
 struct LaunchRecord {
@@ -52,6 +52,8 @@ inline thread_local int g_batch_wide = 0;
 inline thread_local int g_batch_tc_pairs = -1;
 // whether a batch's projections start in one launch with the residual of the guess (fused_start_kernel)
 inline thread_local bool g_batch_fused_start = false;
+// while recording: half the height of a column walk's chunk for every member (sweep_column.cuh), or 0 for the tile sweep
+inline thread_local int g_batch_column = 0;
 // launch a step kernel with programmatic stream serialization (see pdl_wait); inside a stream capture this makes
 // the graph edge to the previous kernel a programmatic one
 template <class... KArgs, class... Args>
@@ -407,6 +409,7 @@ template <class T> struct MomentumArgs {
     int stage;
     T r, one_minus_r;   // gauge-reset weights
     T nu;
+    T one;              // 1: a sum a + b written as a one + b is never merged with the product behind a or b
 };
 
 // ------------------------------------------------------------------------------------------ start of a projection

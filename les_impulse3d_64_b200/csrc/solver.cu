@@ -30,6 +30,7 @@
 #include "sweep_march.cuh"
 #include "sweep_tile.cuh"
 #include "sweep_pair.cuh"
+#include "sweep_column.cuh"
 #include "outputs.cuh"
 #include "setup.h"
 
@@ -197,6 +198,9 @@ template <class T> class Solver : public SolverBase {
     // the FP32 tile sweep with two cells per thread in packed arithmetic (sweep_pair.cuh): the same tile, 256 threads
     static constexpr int kPairNT = 256;
     using PairG = TileGeom<kTileTY, kTileTZ, kPairNT, true>;
+    // and its walk up columns (sweep_column.cuh), 16 x 16 columns of cells per CTA, one CTA per SM
+    static constexpr int kColTX = 16, kColTY = 16;
+    using ColumnG = ColumnGeom<kColTX, kColTY>;
     // the z-march sweep (sweep_march.cuh): 32 x 8 columns of cells per CTA
     static constexpr int kMarchTX = 32, kMarchTY = 8;
     using MarchG = MarchGeom<kMarchTX, kMarchTY>;
@@ -1066,6 +1070,7 @@ private:
         a.r = (T)c_.reinit_r;
         a.one_minus_r = (T)(1.0 - c_.reinit_r);
         a.nu = (T)c_.nu;
+        a.one = T(1);
         if (sweep_kind_ == kSweepMarch) {
             using G = MarchG;
             const dim3 grid((nx_ + G::TX - 1) / G::TX, (ny_ + G::TY - 1) / G::TY, march_chunks());
@@ -1074,6 +1079,13 @@ private:
                                  G::template smem_bytes<T>(), st, a));
         } else if (sweep_kind_ == kSweepPair) {
             if constexpr (sizeof(T) == 4) {
+                if (const int h = column_height()) {
+                    using G = ColumnG;
+                    const dim3 grid((nx_ + G::TX - 1) / G::TX, (ny_ + G::TY - 1) / G::TY, (nz_ + 2 * h - 1) / (2 * h));
+                    if (!record_launch(kLkSweep, kSweepColumn, grid, G::smem_bytes(), a))
+                        check(launch_pdl(sweep_column_kernel<kColTX, kColTY>, grid, dim3(G::NT), G::smem_bytes(), st, a));
+                    return;
+                }
                 const dim3 grid((nx_ + TileG::TX - 1) / TileG::TX, (ny_ + kTileTY - 1) / kTileTY, (nz_ + kTileTZ - 1) / kTileTZ);
                 const size_t smem = PairG::template smem_bytes<T>();
                 if (!record_launch(kLkSweep, kSweepPair, grid, smem, a))
@@ -1304,11 +1316,16 @@ private:
             // selects one cell per thread
             if (kind == "pair" || (kind.empty() && sizeof(T) == 4)) sweep_kind_ = sizeof(T) == 4 ? kSweepPair : kSweepTile;
             sweep_forced_ = !kind.empty();
+            const char* col = std::getenv("CAVITY_COLUMN");
+            column_env_ = col && *col ? std::atoi(col) : -1;
             check(cudaFuncSetAttribute(sweep_tile_kernel<T, kTileTY, kTileTZ, kTileNT>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TileG::template smem_bytes<T>()));
             if constexpr (sizeof(T) == 4)
                 check(cudaFuncSetAttribute(sweep_pair_kernel<kTileTY, kTileTZ, kPairNT>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairG::template smem_bytes<T>()));
+            if constexpr (sizeof(T) == 4)
+                check(cudaFuncSetAttribute(sweep_column_kernel<kColTX, kColTY>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ColumnG::smem_bytes()));
             {
                 const int smem = (int)MarchG::template smem_bytes<T>();
                 check(cudaFuncSetAttribute(sweep_march_kernel<T, kMarchTX, kMarchTY>,
@@ -1395,6 +1412,56 @@ private:
     int march_per_sm_ = 1;
     // z-chunks of a march sweep launch: as many as fill the device's resident CTA slots once (all cavities of a
     // batch together) with at least four layers per chunk; CAVITY_MARCH_CHUNKS overrides
+    // Half the height of a column walk's chunk for a launch over these grids (sweep_column.cuh), or 0 where the tile
+    // sweep is the faster of the two; their results are the same bit for bit.  The walk's time goes as the layer pairs
+    // that an SM walks for the CTAs it runs one after the other (one fits), three of them before each chunk; the tile's
+    // as the CTAs it runs two at a time.  Measured, us per sweep at the chosen height: walk 567 (256^3: 245 layer pairs),
+    // 122 (164 x 164 x 93: 50), 92 (128^3: 35), 100 (seven 64^3: 35), 45 (96^3: 15), 33 (64 x 64 x 128: 11), so 7 + 2.3
+    // to 2.4 each; tile 810 (56 waves), 156 (14), 110 (7), 109 (7), 51 (3), 36 (2), so 5 + 15 each.  One 64^3 grid (7
+    // layer pairs or one wave) stays with the tile.
+    static int column_height(const std::vector<const Solver*>& grids, int sms) {
+        if (sizeof(T) != 4 || grids.empty()) return 0;
+        const int forced = grids[0]->column_env_;
+        if (forced == 0) return 0;
+        int top = 1;
+        bool same = true;
+        long long tiles = 0;
+        for (const Solver* s : grids) {
+            top = std::max(top, s->nz_);
+            same = same && s->nx_ == grids[0]->nx_ && s->ny_ == grids[0]->ny_ && s->nz_ == grids[0]->nz_;
+            tiles += (long long)((s->nx_ + TileG::TX - 1) / TileG::TX) * ((s->ny_ + kTileTY - 1) / kTileTY) *
+                     ((s->nz_ + kTileTZ - 1) / kTileTZ);
+        }
+        if (forced > 0) return std::min(ColumnG::HMAX, (top + 2 * forced - 1) / (2 * forced));
+        int best = 0;
+        long long cost = 50 + (tiles + 2 * sms - 1) / (2 * sms) * 150;
+        std::vector<long long> sm;                    // heap: when each SM is free, the earliest first
+        for (int h = std::min(ColumnG::HMAX, (top + 1) / 2); h >= 3; h--) {
+            long long pairs = 0;                      // layer pairs until the last CTA is done
+            sm.assign(sms, 0);
+            for (const Solver* s : grids) {
+                const int chunks = (s->nz_ + 2 * h - 1) / (2 * h), walk = (s->nz_ + 2 * chunks - 1) / (2 * chunks) + 3;
+                long long ctas = (long long)((s->nx_ + kColTX - 1) / kColTX) * ((s->ny_ + kColTY - 1) / kColTY) * chunks;
+                if (same) {
+                    pairs = (ctas * (long long)grids.size() + sms - 1) / sms * walk;
+                    break;
+                }
+                for (; ctas > 0; ctas--) {
+                    std::pop_heap(sm.begin(), sm.end(), std::greater<long long>());
+                    sm.back() += walk;
+                    pairs = std::max(pairs, sm.back());
+                    std::push_heap(sm.begin(), sm.end(), std::greater<long long>());
+                }
+            }
+            if (70 + 24 * pairs < cost) {
+                cost = 70 + 24 * pairs;
+                best = h;
+            }
+        }
+        return best;
+    }
+    int column_height() const { return g_launch_record ? g_batch_column : column_height({this}, sms_); }
+    int column_env_ = -1;               // CAVITY_COLUMN: 0 the tile, n > 0 the walk in about n z-chunks; -1: the rule
     unsigned int march_chunks() const {
         const long long tiles = (long long)((nx_ + kMarchTX - 1) / kMarchTX) * ((ny_ + kMarchTY - 1) / kMarchTY) *
                                 std::max(g_launch_batch, 1);
@@ -1514,6 +1581,9 @@ public:
             long long cells = (long long)(capacity - (int)m_.size()) * f.n_cell_;
             for (const S_* s : m_) cells += s->n_cell_;
             fused_start_ = cells <= S_::kFusedStartCells;
+            std::vector<const S_*> grids(m_.begin(), m_.end());
+            grids.resize(capacity, &f);           // empty slots take cavities of the first one's grid
+            column_ = S_::column_height(grids, f.sms_);
         }
         proto_ = m_[0];
         par_ = m_[0]->par_;
@@ -1534,6 +1604,9 @@ public:
         check(cudaFuncSetAttribute(sweep_march_batched<T, S_::kMarchTX, S_::kMarchTY>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)S_::MarchG::template smem_bytes<T>()));
+        if constexpr (sizeof(T) == 4)
+            check(cudaFuncSetAttribute(sweep_column_batched<S_::kColTX, S_::kColTY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)S_::ColumnG::smem_bytes()));
         if constexpr (sizeof(T) == 4)
             check(cudaFuncSetAttribute(sweep_pair_batched<kTY, kTZ, S_::kPairNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)S_::PairG::template smem_bytes<T>()));
@@ -1667,7 +1740,7 @@ public:
             for (int S = 0; S < 2; S++) {
                 std::vector<LaunchRecord> rec;
                 {
-                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_);
+                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_, column_);
                     record_member(*s, S ^ d_[slot], S);
                 }
                 const Layout& L = layout_[S];
@@ -1693,7 +1766,7 @@ public:
 private:
     struct RecordGuard {
         RecordGuard(std::vector<LaunchRecord>* r, int batch, int dgemm_tile, int pairs, int tc_pairs, bool fused_start,
-                    int wide) {
+                    int wide, int column) {
             g_launch_record = r;
             g_launch_batch = batch;
             g_dgemm_tile = dgemm_tile;
@@ -1701,6 +1774,7 @@ private:
             g_batch_tc_pairs = tc_pairs;
             g_batch_fused_start = fused_start;
             g_batch_wide = wide;
+            g_batch_column = column;
         }
         ~RecordGuard() {
             g_launch_record = nullptr;
@@ -1710,6 +1784,7 @@ private:
             g_batch_tc_pairs = -1;
             g_batch_fused_start = false;
             g_batch_wide = 0;
+            g_batch_column = 0;
         }
     };
     static size_t align256(size_t n) { return (n + 255) / 256 * 256; }
@@ -1768,7 +1843,7 @@ private:
         const size_t B = m_.size();
         std::vector<std::vector<LaunchRecord>> recs(B);
         for (size_t b = 0; b < B; b++) {
-            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_);
+            RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_, column_);
             if (m_[b]) fn(*m_[b], (int)b);
             else fn(*proto_, 0);
         }
@@ -1826,7 +1901,11 @@ private:
             if (r.variant == kSweepMarch)
                 check(launch_pdl(sweep_march_batched<T, S_::kMarchTX, S_::kMarchTY>, g, dim3(S_::MarchG::NT), r.smem, st,
                                  (const MomentumArgs<T>*)d, items, live));
-            else if (r.variant == kSweepPair) {
+            else if (r.variant == kSweepColumn) {
+                if constexpr (sizeof(T) == 4)
+                    check(launch_pdl(sweep_column_batched<S_::kColTX, S_::kColTY>, g, dim3(S_::ColumnG::NT), r.smem, st,
+                                     (const MomentumArgs<T>*)d, items, live));
+            } else if (r.variant == kSweepPair) {
                 if constexpr (sizeof(T) == 4)
                     check(launch_pdl(sweep_pair_batched<kTY, kTZ, S_::kPairNT>, g, dim3(S_::kPairNT), r.smem, st,
                                      (const MomentumArgs<T>*)d, items, live));
@@ -1992,6 +2071,7 @@ private:
     std::vector<unsigned char> host_[2];      // host copies of the argument buffers
     Layout layout_[2];
     bool mixed_sizes_ = false;
+    int column_ = 0;            // half the height of the column walk's chunks (g_batch_column)
     int wide_ = 0;              // the phases of the paired pass that run the streamed kernel (g_batch_wide)
     int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 128 cells)
     bool loops_ = false;        // conditional refinement loops in the graphs

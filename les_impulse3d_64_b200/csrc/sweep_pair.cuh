@@ -6,7 +6,8 @@
 // (fma.rn.f32x2 and friends, through __ffma2_rn / __fadd2_rn / __fmul2_rn): one instruction does the arithmetic of
 // both cells.  The table values of the y and z axes, the same for both cells, are read once per pair, and the
 // x-neighbours the two cells share are read once.  The expressions and the order of every sum are the tile
-// kernel's (backend.cu:141-330).
+// kernel's (backend.cu:141-330).  Where a sum could be merged with the product behind one of its terms, the code says
+// which rounding is meant (fma2, or a sum through `one`), so that the column walk (sweep_column.cuh) gives the same bits.
 #pragma once
 #include "sweep_tile.cuh"
 
@@ -43,13 +44,13 @@ __device__ __forceinline__ F2 viscous_rk_pair(const MomentumArgs<float>& a, cons
     const Params& p = a.p;
     const F2 cc = ld2(mb);
     const F2 zero = f2(0.f);
-    F2 lap = zero;
+    F2 lap;
     auto tx2 = [&](int k, int i) { return f2(tX(k, i), tX(k, i + 1)); };
     // axis X: the cells' own values differ across the pair
     {
         const F2 up = ld2(mb + 1), dn = ld2(mb - 1);
         if (A == X) {
-            lap = lap + fms2(up - cc, tx2(kInvW, x), cc - dn, tx2(kInvW, x - 1)) * tx2(kInvSp, x);
+            lap = fms2(up - cc, tx2(kInvW, x), cc - dn, tx2(kInvW, x - 1)) * tx2(kInvSp, x);
         } else {
             const bool ha = x < p.nx - 1, hb = x + 1 < p.nx - 1, la = x > 0;
             F2 hi = sel2(ha, hb, (up - cc) * tx2(kInvSp, x + 1), zero);
@@ -57,7 +58,7 @@ __device__ __forceinline__ F2 viscous_rk_pair(const MomentumArgs<float>& a, cons
             if (x == 0) lo = f2(wall.v.x * tX(kInvSp, 0), lo.v.y);
             if (x == p.nx - 1) hi = f2(-wall.v.x * tX(kInvSp, p.nx), hi.v.y);
             if (x + 1 == p.nx - 1) hi = f2(hi.v.x, -wall.v.y * tX(kInvSp, p.nx));
-            lap = lap + (hi - lo) * tx2(kInvW, x);
+            lap = (hi - lo) * tx2(kInvW, x);
         }
     }
     // axes Y and Z: the same index for both cells
@@ -68,7 +69,7 @@ __device__ __forceinline__ F2 viscous_rk_pair(const MomentumArgs<float>& a, cons
         const int s = t == 1 ? MW : MW * MH;
         const F2 up = ld2(mb + s), dn = ld2(mb - s);
         if (t == A) {
-            lap = lap + ((up - cc) * f2(tb(kInvW, q)) - (cc - dn) * f2(tb(kInvW, q - 1))) * f2(tb(kInvSp, q));
+            lap = fma2((up - cc) * f2(tb(kInvW, q)) - (cc - dn) * f2(tb(kInvW, q - 1)), f2(tb(kInvSp, q)), lap);
             continue;
         }
         F2 hi = q < n - 1 ? (up - cc) * f2(tb(kInvSp, q + 1)) : zero;
@@ -82,10 +83,10 @@ __device__ __forceinline__ F2 viscous_rk_pair(const MomentumArgs<float>& a, cons
                 hi = -wall * f2(tb(kInvSp, n));
             }
         }
-        lap = lap + (hi - lo) * f2(tb(kInvW, q));
+        lap = fma2(hi - lo, f2(tb(kInvW, q)), lap);
     }
     F2 val = fma2(f2(dt), fma2(f2(a.nu), lap, L), cc);
-    if (a.stage > 0) val = f2((float)sc.a0) * base + f2((float)sc.b) * val;
+    if (a.stage > 0) val = fma2(f2((float)sc.a0), base, f2((float)sc.b) * val);
     return val;
 }
 
@@ -117,6 +118,8 @@ __device__ void sweep_pair_body(const MomentumArgs<float>& a, const Blk& blk) {
     const T eighth = T(0.125);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int px = 2 * (lane & 15);                          // the pair's first cell within the tile row
+    const F2 one = f2(a.one);
+    auto sum = [&](F2 p0, F2 p1) { return fma2(p0, one, p1); };
     auto kidx = [&](int ix, int iy, int iz) { return (iz * (TY + 1) + iy) * (TX + 1) + ix; };
     auto tx2 = [&](int k, int i) { return f2(tX(k, i), tX(k, i + 1)); };
     // stencil weights of an edge: A per cell (pair), B shared (scalar)
@@ -238,11 +241,11 @@ __device__ void sweep_pair_body(const MomentumArgs<float>& a, const Blk& blk) {
                 const F2 wo = w3s(tZ(kL3, e), l3x) * fms2(uh - ul, f2(tZ(kInvNd3, e)), wh - wl, i3x);
                 return -(wo * fma2(e3l, wl, e3h * wh));
             };
-            F2 L = fma2(half, pz1(1) + uZ0, half * (uY1 + uY0));
+            F2 L = fma2(half, sum(pz1(1), uZ0), half * sum(uY1, uY0));
             if (o4) {
                 const F2 c3 = tx2(kC3, x);
-                L = fma2(c3, pz3(2) + pz3(-1), L);
-                L = fma2(c3, py3(2) + py3(-1), L);
+                L = fma2(c3, sum(pz3(2), pz3(-1)), L);
+                L = fma2(c3, sum(py3(2), py3(-1)), L);
             }
             L = fma2(ld2(Kc + kidx(px, ry + 1, rz + 1)) - kc, tx2(kInvSp, x), L);
             const F2 val = viscous_rk_pair<X, MW, MH>(a, MX + mo, ld2(pu), sc, dt, lidv, x, y, z, bu, L, tX, tY, tZ);
@@ -284,11 +287,11 @@ __device__ void sweep_pair_body(const MomentumArgs<float>& a, const Blk& blk) {
                     const F2 wo = f2(-((l3y * tZ(kL3, e)) * eighth)) * fms2(wh - wl, f2(i3y), vh - vl, f2(tZ(kInvNd3, e)));
                     return wo * fma2(e3l, wl, e3h * wh);
                 };
-                F2 L = fma2(half, pz1(1) + vZ0, half * (vX1 + vX0));
+                F2 L = fma2(half, sum(pz1(1), vZ0), half * sum(vX1, vX0));
                 if (o4) {
                     const F2 c3 = f2(tY(kC3, y));
-                    L = fma2(c3, pz3(2) + pz3(-1), L);
-                    L = fma2(c3, px3(2) + px3(-1), L);
+                    L = fma2(c3, sum(pz3(2), pz3(-1)), L);
+                    L = fma2(c3, sum(px3(2), px3(-1)), L);
                 }
                 L = fma2(ld2(Kc + kidx(px + 1, ry, rz + 1)) - kc, f2(tY(kInvSp, y)), L);
                 const F2 val = viscous_rk_pair<Y, MW, MH>(a, MY + mo, ld2(pv), sc, dt, lidv, x, y, z, bv, L, tX, tY, tZ);
@@ -341,11 +344,11 @@ __device__ void sweep_pair_body(const MomentumArgs<float>& a, const Blk& blk) {
                     const F2 wo = w3s(l3z, tx2(kL3, e)) * fms2(uh - ul, f2(i3z), wh - wl, tx2(kInvNd3, e));
                     return wo * fma2(e3l, ul, e3h * uh);
                 };
-                F2 L = fma2(half, px1(1) + wX0, half * (py1(1) + wY0));
+                F2 L = fma2(half, sum(px1(1), wX0), half * sum(py1(1), wY0));
                 if (o4) {
                     const F2 c3 = f2(tZ(kC3, z));
-                    L = fma2(c3, px3(2) + px3(-1), L);
-                    L = fma2(c3, py3(2) + py3(-1), L);
+                    L = fma2(c3, sum(px3(2), px3(-1)), L);
+                    L = fma2(c3, sum(py3(2), py3(-1)), L);
                 }
                 L = fma2(ld2(Kc + kidx(px + 1, ry + 1, rz)) - kc, f2(tZ(kInvSp, z)), L);
                 const F2 val = viscous_rk_pair<Z, MW, MH>(a, MZ + mo, ld2(pw), sc, dt, lidv, x, y, z, bw, L, tX, tY, tZ);

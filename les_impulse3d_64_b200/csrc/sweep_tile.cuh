@@ -64,6 +64,11 @@ template <class T> __device__ __forceinline__ void st_out(T* p, T v) {
     else asm volatile("st.global.f32 [%0], %1;" ::"l"(g), "f"(v));
 }
 
+// a product rounded by itself: with an explicit fma around it, the sum of two products rounds in the one way that the
+// column walk's packed form rounds it (sweep_column.cuh)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async_elem(void* smem_dst, const void* src) {
     const unsigned int dst = (unsigned int)__cvta_generic_to_shared(smem_dst);
@@ -110,7 +115,7 @@ __device__ __forceinline__ void blend_box(T* mb, const T* vb, int uoff, T r, T o
     for (int e = threadIdx.x; e < MC * MH * MD; e += NT) {
         const int ix = e % MC, iy = (e / MC) % MH, iz = e / (MC * MH);
         const int i = (iz * MH + iy) * MW + ix;
-        mb[i] = r * mb[i] + omr * vb[uoff + iz * VP + iy * VW + ix];
+        mb[i] = fma(r, mb[i], mul_rn(omr, vb[uoff + iz * VP + iy * VW + ix]));
     }
 }
 
@@ -256,8 +261,8 @@ __device__ bool tile_prologue(const MomentumArgs<T>& a, const Blk& blk, const Ti
         const T* v0 = SV + ((iz + 2) * VH + iy) * VW + 2 + ix;
         const T* w0 = SW + (iz * WH + iy + 2) * WW + 2 + ix;
         const int mi = (iz * MH + iy) * MW + ix;
-        Kc[e] = T(0.5) * ((u0[0] * MX[mi] + u0[1] * MX[mi + 1]) + (v0[0] * MY[mi] + v0[VW] * MY[mi + MW]) +
-                          (w0[0] * MZ[mi] + w0[WP] * MZ[mi + MH * MW]));
+        Kc[e] = T(0.5) * (fma(u0[0], MX[mi], mul_rn(u0[1], MX[mi + 1])) + fma(v0[0], MY[mi], mul_rn(v0[VW], MY[mi + MW])) +
+                          fma(w0[0], MZ[mi], mul_rn(w0[WP], MZ[mi + MH * MW])));
     }
     __syncthreads();
     return true;
