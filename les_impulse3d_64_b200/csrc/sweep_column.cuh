@@ -21,14 +21,14 @@
 //
 // What bounds the tile sweep is the L1 data pipe and instruction issue (1,220 thread instructions per cell, 72% of the
 // pipe): each face evaluates its wide edges itself, and a tile stages 3.4 velocities per cell and component.  The walk
-// issues 580 per cell and reads a staged pair once per edge.  16 x 16 columns are the most that leave a thread its 160
+// issues 626 per cell and reads a staged pair once per edge.  16 x 16 columns are the most that leave a thread its 160
 // registers (12 warps; 32 x 8 have 1.50 columns per useful one, these 1.41), and a pair holds layers of two half chunks
 // because the pair's halves then share every x and y table value.  Tables stay in shared memory, in both halves: as
 // register pairs they spilled (128^3, one sweep 130 us, so 117).  The branches on the order, on walls and on the layers
 // before the chunk are compile-time and a layer's stores come after its loads, so the loads overlap (117 us, so 99).
 // Measured against the tile sweep, us per sweep: 256^3 567 and 810, 164 x 164 x 93 122 and 156, 128^3 92 and 110, 96^3
 // 45 and 51, 64 x 64 x 128 33 and 36, seven 64^3 100 and 109.  What bounds it now is the latency of shared-memory reads
-// with three warps on a scheduler (issue 50%, data pipe 57%).
+// with three warps on a scheduler (issue 50%, data pipe 51%).
 //
 // The expressions and the order of every sum are sweep_pair.cuh's, so the results are its results bit for bit (a sign
 // that it applies to a product is applied here to the factor or to the sum, which rounds the same).
