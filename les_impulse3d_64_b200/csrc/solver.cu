@@ -1437,21 +1437,29 @@ private:
         long long cost = 50 + (tiles + 2 * sms - 1) / (2 * sms) * 150;
         std::vector<long long> sm;                    // heap: when each SM is free, the earliest first
         for (int h = std::min(ColumnG::HMAX, (top + 1) / 2); h >= 3; h--) {
-            long long pairs = 0;                      // layer pairs until the last CTA is done
-            sm.assign(sms, 0);
+            auto chunks = [&](const Solver* s) { return (s->nz_ + 2 * h - 1) / (2 * h); };
+            auto walk = [&](const Solver* s) { return (s->nz_ + 2 * chunks(s) - 1) / (2 * chunks(s)) + 3; };
+            auto ctas = [&](const Solver* s) {
+                return (long long)((s->nx_ + kColTX - 1) / kColTX) * ((s->ny_ + kColTY - 1) / kColTY) * chunks(s);
+            };
+            long long pairs = 0, all = 0, work = 0;   // layer pairs until the last CTA is done; CTAs, their layer pairs
             for (const Solver* s : grids) {
-                const int chunks = (s->nz_ + 2 * h - 1) / (2 * h), walk = (s->nz_ + 2 * chunks - 1) / (2 * chunks) + 3;
-                long long ctas = (long long)((s->nx_ + kColTX - 1) / kColTX) * ((s->ny_ + kColTY - 1) / kColTY) * chunks;
-                if (same) {
-                    pairs = (ctas * (long long)grids.size() + sms - 1) / sms * walk;
-                    break;
-                }
-                for (; ctas > 0; ctas--) {
-                    std::pop_heap(sm.begin(), sm.end(), std::greater<long long>());
-                    sm.back() += walk;
-                    pairs = std::max(pairs, sm.back());
-                    std::push_heap(sm.begin(), sm.end(), std::greater<long long>());
-                }
+                all += ctas(s);
+                work += ctas(s) * walk(s);
+            }
+            if (same) {
+                pairs = (all + sms - 1) / sms * walk(grids[0]);
+            } else if (all > 8LL * sms) {             // many rounds: the SMs end together but for part of a walk
+                pairs = work / sms + (h + 3) / 2;
+            } else {
+                sm.assign(sms, 0);
+                for (const Solver* s : grids)
+                    for (long long k = ctas(s); k > 0; k--) {
+                        std::pop_heap(sm.begin(), sm.end(), std::greater<long long>());
+                        sm.back() += walk(s);
+                        pairs = std::max(pairs, sm.back());
+                        std::push_heap(sm.begin(), sm.end(), std::greater<long long>());
+                    }
             }
             if (70 + 24 * pairs < cost) {
                 cost = 70 + 24 * pairs;
