@@ -278,7 +278,6 @@ public:
     void step_async(int count) override {
         if (auto_tune_ && tune_.ms == 0 && pending_.empty()) autotune(6, nullptr, nullptr, nullptr, nullptr);
         ensure_graphs(false);
-        if (pending_.empty()) steps_before_ = hc_.steps;
         if (!tail_host_) {
             const size_t off = 256 * ((sizeof(Control) + 255) / 256);
             check(cudaHostAlloc(&tail_host_, off + sizeof(float) * 16, cudaHostAllocMapped));
@@ -286,17 +285,21 @@ public:
         }
         probes_fresh_ = false;
         for (int i = 0; i < count; i++) {
-            if (eager_) enqueue_step(par_, false, true);
-            else check(cudaGraphLaunch(exec_[par_], stream_));
-            // the parity flips only when the step succeeds; sync() checks that for the queued steps
-            pending_.push_back({par_});
-            par_ ^= 1;
+            queue_step(false);
             char* d = static_cast<char*>(tail_dev_);
             step_tail_kernel<T><<<1, 32, 0, stream_>>>(out_args(), probe_cells_, c_.n_probes,
                                                        reinterpret_cast<float*>(d + 256 * ((sizeof(Control) + 255) / 256)),
                                                        ctrl_, reinterpret_cast<Control*>(d));
         }
         tail_queued_ = true;
+    }
+    // queue one step; the parity flips only when it succeeds: sync() checks that for the queued steps
+    void queue_step(bool timing) {
+        if (pending_.empty()) steps_before_ = hc_.steps;
+        if (eager_) enqueue_step(par_, timing, true);
+        else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[par_], stream_));
+        pending_.push_back({par_});
+        par_ ^= 1;
     }
     void sync(CavityReport* r) override {
         settle();
@@ -339,6 +342,7 @@ public:
         if (!pending_.empty() && !batch_pending_) settle();
     }
     void resume_stalled() {
+        stalls_++;
         loops_ = true;
         drop_graphs();
         tail_queued_ = false;
@@ -671,9 +675,10 @@ public:
     }
     long long pressure_passes() const override { return hc_.pass_count; }
 
-    // `steps` steps through the plain step graph, each timed by events around its launch; then, when `kms` is
-    // given, `steps` more through the graph with events around the kernels (they cost launch latency, so the step
-    // times come from the plain graph), for the per-kernel times
+    // `steps` steps through the plain step graph, each timed by events around its launch, or to the end of the host's
+    // part where it stalls; then, when `kms` is given, `steps` more through the graph with events around the kernels (they
+    // cost launch latency, so the step times come from the plain graph), for the per-kernel times.  That graph holds the
+    // refinement loops, so its steps never stall.
     void time_steps(int warmup, int steps, int flush, float* ms, float* kms) override {
         probes_fresh_ = false;
         if (flush && !flush_) check(cudaMalloc(&flush_, kFlushBytes));
@@ -681,22 +686,23 @@ public:
         ensure_graphs(false);
         if (kms) ensure_graphs(true);
         for (double& t : timed_ms_) t = 0;
-        cudaEvent_t e0, e1;
-        check(cudaEventCreate(&e0));
-        check(cudaEventCreate(&e1));
+        TimingEvents ev;
         for (int pass = 0; pass < (kms ? 2 : 1); pass++) {
             const bool timing = pass == 1;
             for (int i = 0; i < steps; i++) {
+                ensure_graphs(timing);                   // a step that stalls drops them
                 if (flush) check(cudaMemsetAsync(flush_, i & 0xff, kFlushBytes, stream_));
-                check(cudaEventRecord(e0, stream_));
-                if (eager_) enqueue_step(par_, timing, true);
-                else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[par_], stream_));
-                pending_.push_back({par_});
-                par_ ^= 1;
-                check(cudaEventRecord(e1, stream_));
+                const long long stalls = stalls_;
+                check(cudaEventRecord(ev.begin, stream_));
+                queue_step(timing);
+                check(cudaEventRecord(ev.end, stream_));
                 sync(nullptr);
                 if (!timing) {
-                    check(cudaEventElapsedTime(&ms[i], e0, e1));
+                    if (stalls_ != stalls) {
+                        check(cudaEventRecord(ev.end, stream_));
+                        check(cudaEventSynchronize(ev.end));
+                    }
+                    check(cudaEventElapsedTime(&ms[i], ev.begin, ev.end));
                     continue;
                 }
                 for (int kind = 0; kind < kNumTimed; kind++) {
@@ -711,8 +717,6 @@ public:
                 }
             }
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
     }
 
     // Time whole steps under each candidate launch shape from the current state, restore the state after each,
@@ -822,6 +826,17 @@ public:
 
 private:
     static constexpr size_t kFlushBytes = 256ull << 20;
+    struct TimingEvents {
+        cudaEvent_t begin = nullptr, end = nullptr;
+        TimingEvents() {
+            check(cudaEventCreate(&begin));
+            check(cudaEventCreate(&end));
+        }
+        ~TimingEvents() {
+            cudaEventDestroy(begin);
+            cudaEventDestroy(end);
+        }
+    };
 
     // ------------------------------------------------------------------------------ set-up
     void setup_params() {
@@ -1162,12 +1177,9 @@ private:
         launch_transforms(st, phi, h, use_h);
         launch_residual(st, phi, h, use_h);
     }
-    // the passes of a step's graph without a loop: one, or two on the tensor cores, the last of which may stall the step;
-    // `t0`, `t1`: events around the first pass's transforms
-    void launch_passes(cudaStream_t st, double* phi, int stage, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = nullptr) {
-        if (t0) check(cudaEventRecordWithFlags(t0, st, cudaEventRecordExternal));
+    // the passes of a step's graph without a loop: one, or two on the tensor cores, the last of which may stall the step
+    void launch_passes(cudaStream_t st, double* phi, int stage) {
         launch_transforms(st, phi, 0, 0);
-        if (t1) check(cudaEventRecordWithFlags(t1, st, cudaEventRecordExternal));
         launch_residual(st, phi, 0, 0, 0, !tc_fdm_, stage);
         if (!tc_fdm_) return;
         launch_transforms(st, phi, 0, 0);
@@ -1205,8 +1217,8 @@ private:
         if (!record_launch(kLkFinish, 0, grid, 0, a)) check(launch_pdl(finish_kernel<T>, grid, dim3(kThreads), 0, st, a));
     }
 
-    // A pressure refinement loop inside a stream capture (loops_): one pass, then a conditional while-node whose body is
-    // one pass.  `first_residual` launches the kernels that set the loop condition before them.
+    // A pressure refinement loop inside a stream capture (loops_, and the timing graphs): one pass, then a conditional
+    // while-node whose body is one pass.  `first_residual` launches the kernels that set the loop condition before them.
     template <class F>
     void captured_loop(F first_residual, double* phi, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = nullptr) {
         cudaStreamCaptureStatus status;
@@ -1275,15 +1287,14 @@ private:
             if (timing) mark(after_start, true);
             pull_control();
             continue_passes(timing, stage);
-        } else if (loops_) {
+        } else if (loops_ || timing) {
             captured_loop([&](cudaGraphConditionalHandle h) {
                 launch_start(stream_, M_[out], true, stage, S, cur, h, 1, between);
                 if (timing) mark(after_start, false);
             }, phi, t0, t1);
         } else {
-            launch_start(stream_, M_[out], true, stage, S, cur, 0, 0, between);
-            if (timing) mark(after_start, false);
-            launch_passes(stream_, phi, stage, t0, t1);
+            launch_start(stream_, M_[out], true, stage, S, cur, 0, 0);
+            launch_passes(stream_, phi, stage);
         }
         finish_stage(S, stage, timing, eager);
     }
@@ -1488,6 +1499,7 @@ private:
     std::vector<Pending> pending_;
     bool batch_pending_ = false;        // queued by a batch
     bool loops_ = false;                // step graphs with conditional refinement loops (after a stalled solve)
+    long long stalls_ = 0;              // stalled steps that the host finished
     long long steps_before_ = 0;
     // fields: three buffer sets of velocity, impulse and potential (state, stage outputs)
     T* U_[3][3];

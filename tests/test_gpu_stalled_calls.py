@@ -1,0 +1,57 @@
+"""The calls around a solve that stalls, that is, needs more pressure passes than the step's graph runs (Solver::settle):
+each leaves the cavity where the same steps leave one that runs kernel by kernel (CAVITY_GRAPHS=0), whose refinement loop
+the host drives anyway.  Two forms stall in their first step: the tensor-core transforms (two passes a solve) above 2^18
+cells, where the projection starts in two launches, and the FP64 ones (one pass) in one launch."""
+import numpy as np
+import pytest
+
+from les_impulse3d_64_b200 import workloads
+from les_impulse3d_64_b200.api import Cavity
+
+pytestmark = pytest.mark.gpu
+FIELDS = ('u', 'v', 'w', 'mx', 'my', 'mz', 'phi')
+# precision, CAVITY_FDM, passes a solve that the graph runs, cells along x and y, along z, tolerance
+FORMS = {'tc': ('mixed', 'tc', 2, 72, 64, 1e-14), 'fp64': ('fp64', '', 1, 64, 64, 3e-15)}
+
+
+def make(form, monkeypatch, eager=False, seed=5, **changes):
+    precision, fdm, _, n, nz, rtol = FORMS[form]
+    monkeypatch.setenv('CAVITY_FDM', fdm)
+    if eager:
+        monkeypatch.setenv('CAVITY_GRAPHS', '0')
+    s = workloads.settings(n, 400.0, nz=nz, beta=1.5, cfl=0.5, **{'fdm_rtol': rtol, **changes})
+    cav = Cavity(s, precision=precision)
+    monkeypatch.delenv('CAVITY_GRAPHS', raising=False)
+    cav.initialize(*workloads.initial_noise(cav.shapes, 1e-2, seed))
+    return cav
+
+
+def stalling_step(cav, form):
+    """One step of a kernel-by-kernel cavity; its solves take more passes than the graph of a step runs."""
+    before = cav.pressure_passes()
+    cav.step()
+    assert cav.pressure_passes() - before > 3 * FORMS[form][2]
+
+
+def assert_same(a, b):
+    assert a.report() == b.report()
+    for k in FIELDS:
+        assert np.array_equal(a.field(k), b.field(k)), k
+
+
+@pytest.mark.parametrize('form', FORMS)
+def test_time_steps(form, monkeypatch):
+    """The first timed step stalls: the steps go on, and its time runs to the end of the host's part."""
+    timed, eager = make(form, monkeypatch), make(form, monkeypatch, eager=True)
+    try:
+        ms, kms = timed.time_steps(0, 3, flush_l2=False)
+        stalling_step(eager, form)
+        for _ in range(5):
+            eager.step()
+        assert_same(timed, eager)
+        assert ms[0] > 0.8 * ms[1:].min() > 0 and kms.min() > 0
+        times = timed.kernel_times()
+        assert all(times[k] > 0 for k in ('sweep', 'projection_start', 'finish', 'transforms'))
+    finally:
+        timed.close()
+        eager.close()
