@@ -734,36 +734,37 @@ public:
         void* saved = nullptr;
         check(cudaMalloc(&saved, (size_t)bytes));
         checkpoint_save(saved, 1);
-        cudaEvent_t e0, e1;
-        check(cudaEventCreate(&e0));
-        check(cudaEventCreate(&e1));
+        TimingEvents ev;
+        // The time of a step, negative when one fails.  Where a solve stalls (resume_stalled) the candidate is timed again:
+        // its graphs hold the refinement loops then, and a further stall is not possible.
         auto time_candidate = [&](const Tuning& cand) {
             tune_ = cand;
             if (cand.sweep >= 0) sweep_kind_ = cand.sweep;
             drop_graphs();
             float ms = -1;
-            try {
-                ensure_graphs(false);
-                step(nullptr);                                   // warm-up (graph upload)
-                check(cudaEventRecord(e0, stream_));
-                for (int i = 0; i < steps; i++) {
-                    check(cudaGraphLaunch(exec_[par_], stream_));
-                    pending_.push_back({par_});
-                    par_ ^= 1;
+            if (eager_) return ms;
+            for (bool again = true; again;) {
+                again = false;
+                try {
+                    step(nullptr);                               // warm-up (graph upload)
+                    ensure_graphs(false);
+                    const long long stalls = stalls_;
+                    check(cudaEventRecord(ev.begin, stream_));
+                    for (int i = 0; i < steps; i++) queue_step(false);
+                    check(cudaEventRecord(ev.end, stream_));
+                    sync(nullptr);
+                    again = stalls_ != stalls;
+                    check(cudaEventElapsedTime(&ms, ev.begin, ev.end));
+                    ms /= steps;
+                } catch (const std::exception&) {
+                    ms = -1;                                     // a failed step: not a candidate
                 }
-                check(cudaEventRecord(e1, stream_));
-                sync(nullptr);
-                check(cudaEventElapsedTime(&ms, e0, e1));
-                ms /= steps;
-            } catch (const std::exception&) {
-                ms = -1;                                         // a failed step: not a candidate
+                pending_.clear();
+                checkpoint_load(saved, 1);
             }
-            pending_.clear();
-            checkpoint_load(saved, 1);
             return ms;
         };
         Tuning best;
-        best.ms = -1;
         auto consider = [&](const Tuning& cand) {
             const float ms = time_candidate(cand);
             if (ms > 0 && (best.ms < 0 || ms < best.ms)) {
@@ -790,9 +791,14 @@ public:
             for (int c : cs) sweeps.push_back(Tuning{c, 0, -1, kSweepMarch, 0});
         }
         if (forced == kSweepFace) sweeps.push_back(Tuning{0, 0, -1, kSweepFace, 0});
-        for (const Tuning& t : sweeps) consider(t);
-        // round 2: the FP64 transforms, with that sweep
-        if (!tc_fdm_ && best.ms > 0) {
+        bool plain;
+        do {
+            plain = !loops_;
+            best = Tuning{};
+            best.ms = -1;
+            for (const Tuning& t : sweeps) consider(t);
+            // round 2: the FP64 transforms, with that sweep
+            if (tc_fdm_ || best.ms <= 0) continue;
             std::vector<std::pair<int, int>> tiles = {{64, kPassSix}, {32, kPassSix}};
             if (fused_pass_capacity() > 0) tiles.push_back({32, kPassOneLaunch});
             if (pair_pass_fits(nx_, ny_, nz_)) tiles.push_back({0, kPassPairs});
@@ -803,9 +809,7 @@ public:
                 cand.fused = t.second;
                 consider(cand);
             }
-        }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        } while (plain && loops_);              // a solve stalled: the first of them were timed without the loops
         cudaFree(saved);
         if (best.ms < 0) best = Tuning{};
         tune_ = best;

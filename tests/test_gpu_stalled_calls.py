@@ -55,3 +55,24 @@ def test_time_steps(form, monkeypatch):
     finally:
         timed.close()
         eager.close()
+
+
+@pytest.mark.parametrize('form', FORMS)
+def test_autotune(form, monkeypatch):
+    """Stalls under the tuner's candidates: none is thrown out or timed over an aborted step, the state comes back, and the
+    tuned cavity steps on as an untuned one (the sweep kernel is fixed: the other choices are bit for bit the same)."""
+    monkeypatch.setenv('CAVITY_SWEEP', 'tile')
+    tuned, eager = make(form, monkeypatch), make(form, monkeypatch, eager=True)
+    try:
+        report = tuned.report()
+        chunks, tile, fused, ms = tuned.autotune(steps=3)
+        assert tuned.report() == report
+        stalling_step(eager, form)
+        assert tuned.step() == eager.report()
+        for _ in range(3):
+            assert tuned.step() == eager.step()
+        assert_same(tuned, eager)
+        assert chunks == 0 and ms > 0.8 * float(tuned.time_steps(2, 8, flush_l2=False)[0].min())
+    finally:
+        tuned.close()
+        eager.close()
