@@ -1669,13 +1669,18 @@ public:
     // Per-step device time (ms, summed over the three stages) of the batch's parts: the sweeps, the projection
     // starts with the residuals of their guesses, the first pressure pass of each stage (transforms and
     // residual), and the finishes, over `steps` steps through a second graph with events between the parts.
-    // The steps advance the cavities as cavity_batch_step_async does (the same kernels in the same order).
+    // The steps advance the cavities as cavity_batch_step_async does (the same kernels in the same order); that graph holds
+    // the refinement loops whether or not the plain one does, so that the first pass stands alone and no step stalls.
     void part_times(int steps, double* ms) override {
         if (queued_) fail("batch: steps are queued; sync first");
         if (!tev_[0])
             for (cudaEvent_t& e : tev_) check(cudaEventCreate(&e));
         drop_timing();
-        for (int S = 0; S < 2; S++) build(S, true);
+        {
+            struct Restore { bool& v; const bool old; ~Restore() { v = old; } } restore{loops_, loops_};
+            loops_ = true;
+            for (int S = 0; S < 2; S++) build(S, true);
+        }
         for (int k = 0; k < kParts; k++) ms[k] = 0;
         for (int i = 0; i < steps; i++) {
             launch_step(texec_);

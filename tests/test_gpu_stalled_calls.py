@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from les_impulse3d_64_b200 import workloads
-from les_impulse3d_64_b200.api import Cavity
+from les_impulse3d_64_b200.api import Batch, Cavity
 
 pytestmark = pytest.mark.gpu
 FIELDS = ('u', 'v', 'w', 'mx', 'my', 'mz', 'phi')
@@ -76,3 +76,26 @@ def test_autotune(form, monkeypatch):
     finally:
         tuned.close()
         eager.close()
+
+
+def test_part_times(monkeypatch):
+    """A batch's parts: the first pass is one pass of the two that a tensor-core graph runs, also on stalling steps, and
+    the steps are ordinary ones.  Its transforms and residual are those that a cavity alone times (within a half)."""
+    member, alone = make('tc', monkeypatch), make('tc', monkeypatch)
+    batch = Batch([member])
+    try:
+        first, second = batch.part_times(2), batch.part_times(2)
+        alone.time_steps(0, 2, flush_l2=False)
+        times = alone.kernel_times()
+        one_pass = times['transforms'] + times['guess_residual']
+        for parts in (first, second):
+            assert 0.5 * one_pass < parts['first_pass'] < 1.5 * one_pass
+        assert all(first[k] > 0.5 * second[k] for k in first)
+        assert member.report()['steps'] == alone.report()['steps'] == 4
+        for k in FIELDS:           # the sums of a batch group their terms by other blocks (1e-6 of the FP32 fields)
+            x, y = member.field(k), alone.field(k)
+            assert np.abs(x - y).max() <= 1e-6 * np.abs(y).max(), k
+    finally:
+        batch.close()
+        member.close()
+        alone.close()
