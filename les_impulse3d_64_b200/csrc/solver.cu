@@ -1675,9 +1675,19 @@ public:
         if (queued_) fail("batch: steps are queued; sync first");
         if (!tev_[0])
             for (cudaEvent_t& e : tev_) check(cudaEventCreate(&e));
+        for (S_* s : m_)
+            if (s && !proto_) proto_ = s;                 // what the empty slots record
+        if (!proto_) fail("batch part times: every slot is empty");
         drop_timing();
         {
-            struct Restore { bool& v; const bool old; ~Restore() { v = old; } } restore{loops_, loops_};
+            struct Restore {
+                Batch* b;
+                const bool loops;
+                ~Restore() {
+                    b->loops_ = loops;
+                    b->proto_ = nullptr;
+                }
+            } restore{this, loops_};
             loops_ = true;
             for (int S = 0; S < 2; S++) build(S, true);
         }
