@@ -332,14 +332,15 @@ public:
     // queued work returns at once, the state it reads being untouched, and the host finishes that step and the queued
     // ones after it here, pass by pass.  From then on the cavity's graphs have the while-nodes (loops_).
     void settle() {
-        check(cudaStreamSynchronize(stream_));
+        if (batch_pending_) check(cudaDeviceSynchronize());       // they run on the batch's stream, which may be gone
+        else check(cudaStreamSynchronize(stream_));
         if (tail_queued_) std::memcpy(&hc_, tail_control(), sizeof hc_);      // written by the last step's tail
         else pull_control();
         if (hc_.error == kStalled) resume_stalled();
     }
-    // before an operation that reads the state while steps may be queued (a batch's steps are settled by its sync)
+    // before an operation that reads the state while steps may be queued
     void settle_queued() {
-        if (!pending_.empty() && !batch_pending_) settle();
+        if (!pending_.empty()) settle();
     }
     void resume_stalled() {
         stalls_++;
@@ -1501,7 +1502,7 @@ private:
         bool statistics = false;
     };
     std::vector<Pending> pending_;
-    bool batch_pending_ = false;        // queued by a batch
+    bool batch_pending_ = false;        // queued by a batch that has not waited for them
     bool loops_ = false;                // step graphs with conditional refinement loops (after a stalled solve)
     long long stalls_ = 0;              // stalled steps that the host finished
     long long steps_before_ = 0;
@@ -1751,6 +1752,7 @@ public:
                 }
                 continue;
             }
+            m_[i]->batch_pending_ = false;
             try {
                 m_[i]->sync(reports ? &reports[i] : nullptr);
             } catch (const std::exception& e) {

@@ -99,3 +99,23 @@ def test_part_times(monkeypatch):
         batch.close()
         member.close()
         alone.close()
+
+
+def test_reading_a_member_before_the_batch_waits(monkeypatch):
+    """A member's getters and its own wait finish its batch's queued steps first, also one that stalls."""
+    a, b = make('tc', monkeypatch), make('tc', monkeypatch)
+    batch = Batch([a, b])
+    try:
+        batch.step_async(3)
+        early = a.field('u')
+        assert b.sync()['steps'] == 3
+        assert [r['steps'] for r in batch.sync()] == [3, 3]
+        assert np.array_equal(early, a.field('u'))
+        for k in FIELDS:
+            assert np.array_equal(a.field(k), b.field(k)), k
+        batch.step_async(2)
+        assert [r['steps'] for r in batch.sync()] == [5, 5]
+    finally:
+        batch.close()
+        a.close()
+        b.close()
