@@ -614,6 +614,9 @@ public:
         check(cudaStreamSynchronize(stream_));
     }
     void set_clock(double t, long long steps, double last_dt) override {
+        settle_queued();
+        steps_before_ += steps - hc_.steps;      // queued steps are counted from it
+        tail_queued_ = false;                    // the tail's copy has the old clock
         hc_.t = t; hc_.steps = steps; hc_.last_dt = last_dt;
         push_control();
         check(cudaStreamSynchronize(stream_));

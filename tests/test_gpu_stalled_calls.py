@@ -119,3 +119,27 @@ def test_reading_a_member_before_the_batch_waits(monkeypatch):
         batch.close()
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize('form', FORMS)
+def test_set_clock_while_steps_are_queued(form, monkeypatch):
+    """The clock is set after the queued steps, the stalled one among them, and the wait reports it."""
+    queued, eager = make(form, monkeypatch), make(form, monkeypatch, eager=True)
+    try:
+        queued.step_async(3)
+        queued.set_clock(7.0, 100, 2e-3)
+        report = queued.sync()
+        assert (report['time'], report['steps'], report['dt']) == (7.0, 100, 2e-3)
+        stalling_step(eager, form)
+        for _ in range(2):
+            eager.step()
+        eager.set_clock(7.0, 100, 2e-3)
+        assert_same(queued, eager)
+        queued.step_async(2)
+        queued.sync()
+        for _ in range(2):
+            eager.step()
+        assert_same(queued, eager)
+    finally:
+        queued.close()
+        eager.close()
