@@ -262,6 +262,10 @@ public:
     // -------------------------------------------------------------------------------- ABI operations
     void initialize(const double* v_noise, const double* w_noise) override {         // backend.cu:1075-1088
         probes_fresh_ = false;
+        settle_queued();
+        pending_.clear();
+        batch_pending_ = false;
+        tail_queued_ = false;
         const double* src[3] = {nullptr, v_noise, w_noise};
         for (int k = 0; k < 3; k++) {
             if (src[k]) check(cudaMemcpyAsync(dstage_[0], src[k], sizeof(double) * size_[k], cudaMemcpyHostToDevice, stream_));

@@ -143,3 +143,21 @@ def test_set_clock_while_steps_are_queued(form, monkeypatch):
     finally:
         queued.close()
         eager.close()
+
+
+@pytest.mark.parametrize('form', FORMS)
+def test_initialize_while_steps_are_queued(form, monkeypatch):
+    """The steps queued before belong to the old state: a stall among those queued after is not taken for one of them."""
+    queued, eager = make(form, monkeypatch), make(form, monkeypatch, eager=True)
+    try:
+        queued.step_async(1)
+        for cav in (queued, eager):
+            cav.initialize(*workloads.initial_noise(cav.shapes, 2e-2, 9))
+        queued.step_async(2)
+        queued.sync()
+        stalling_step(eager, form)
+        eager.step()
+        assert_same(queued, eager)
+    finally:
+        queued.close()
+        eager.close()
