@@ -76,7 +76,10 @@ int cavity_destroy(CavitySolver* s);
 int cavity_initialize(CavitySolver* s, const double* v_noise, const double* w_noise);
 int cavity_step(CavitySolver* s, CavityReport* report);
 /* Enqueue `count` steps without waiting for the GPU; cavity_sync then waits, checks every step's status
- * and fills the report of the last one.  Steps of different handles overlap on the device. */
+ * and fills the report of the last one.  Steps of different handles overlap on the device.
+ * A queued step holds one pressure pass per solve, two on the tensor cores.  Where a solve needs more (a tolerance close
+ * to rounding), the steps queued behind it return at once and the wait (cavity_sync, or a call that reads or sets the
+ * state) finishes the step and runs them again, to the same results. */
 int cavity_step_async(CavitySolver* s, int count);
 int cavity_sync(CavitySolver* s, CavityReport* report);
 int cavity_get_field(CavitySolver* s, int field, void* out);

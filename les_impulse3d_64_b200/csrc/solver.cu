@@ -333,8 +333,8 @@ public:
     // tensor cores, whose FP32 transforms usually take a second): a conditional while-node for the rare further pass cost
     // 9 us per solve even when it ran nothing, the breaks in the chain of programmatic launches included (a step of
     // 32 x 32 x 8 cells 173 us with them, 146 without; 64^3 282 and 256).  A solve that needs more stalls: the rest of the
-    // queued work returns at once, the state it reads being untouched, and the host finishes that step and the queued
-    // ones after it here, pass by pass.  From then on the cavity's graphs have the while-nodes (loops_).
+    // queued work returns at once, the state it reads being untouched, and the host finishes that step here, pass by pass.
+    // From then on the cavity's graphs have the while-nodes (loops_); the steps queued after it run through those.
     void settle() {
         if (batch_pending_) check(cudaDeviceSynchronize());       // they run on the batch's stream, which may be gone
         else check(cudaStreamSynchronize(stream_));
@@ -351,27 +351,27 @@ public:
         loops_ = true;
         drop_graphs();
         tail_queued_ = false;
-        const long long done = hc_.steps - steps_before_;
+        const size_t stalled = (size_t)std::max(hc_.steps - steps_before_, 0LL);
         hc_.error = kOk;
         push_control();
-        for (size_t k = (size_t)std::max(done, 0LL); k < pending_.size(); k++) {
+        for (size_t k = stalled; k < pending_.size(); k++) {
             const Pending q = pending_[k];
-            if ((long long)k == done) {
+            if (k == stalled) {
                 const int stage = hc_.stage;
                 continue_passes(false, stage);
                 finish_stage(q.par, stage, false, true);
                 for (int s = stage + 1; s < 3; s++) enqueue_stage(q.par, s, false, true);
             } else {
-                enqueue_step(q.par, false, true);
+                ensure_graphs(false);
+                check(cudaGraphLaunch(exec_[q.par], stream_));
             }
-            pull_control();
-            if (hc_.error) return;
             if (q.ring >= 0)
                 probes_kernel<T><<<1, 32, 0, stream_>>>(out_args(q.par ^ 1), probe_cells_, c_.n_probes,
                                                         ring_dev_ + (size_t)q.ring * 2 * c_.n_probes);
             if (q.statistics) launch_statistics(q.par ^ 1);
         }
         check(cudaStreamSynchronize(stream_));
+        pull_control();
     }
     void report(CavityReport* r) override {
         r->steps = hc_.steps; r->time = hc_.t; r->dt = hc_.last_dt; r->cfl = hc_.last_cfl;

@@ -161,3 +161,25 @@ def test_initialize_while_steps_are_queued(form, monkeypatch):
     finally:
         queued.close()
         eager.close()
+
+
+def test_failing_step_queued_behind_a_stall(monkeypatch):
+    """The first queued step stalls, the third does not converge: the wait says so as kernel-by-kernel steps do, and both
+    cavities stand at the second step's state, probes and statistics included."""
+    queued, eager = (make('fp64', monkeypatch, eager=e, fdm_rtol=1e-15) for e in (False, True))
+    try:
+        queued.step_outputs_async(4, statistics=True)
+        with pytest.raises(RuntimeError, match='residual .* > FDM_RTOL after 8 passes') as error:
+            queued.sync_outputs()
+        for _ in range(2):
+            eager.step_outputs_async(1, statistics=True)
+            eager.sync_outputs()
+        with pytest.raises(RuntimeError) as same:
+            eager.step()
+        assert str(error.value) == str(same.value)
+        assert_same(queued, eager)
+        assert np.array_equal(queued.probes(), eager.probes())
+        assert np.array_equal(queued.statistics(), eager.statistics())
+    finally:
+        queued.close()
+        eager.close()
