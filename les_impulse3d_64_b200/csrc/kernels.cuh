@@ -119,7 +119,8 @@ struct alignas(16) Control {
     // current pressure solve (backend.cu:816-847)
     double rhs_norm2, res_norm2, phi_sum, rhs_norm, rel;
     int passes, use_rhs, reset_phi, zero_rhs;
-    int cond, stage, pad1, pad2;
+    int cond, stage;
+    int long_solves, pad2;      // solves that took more passes than a step's graph without refinement loops runs
     // warm-start history: last three potential increments (backend.cu:857-873, 929-939)
     double hist_t[3], hist_scale[3];
     int hist_buf[3], hist_count;
@@ -831,8 +832,8 @@ struct ResidualArgs {
     cudaGraphConditionalHandle handle;
     int use_handle;
     int start;                 // 1: residual of the warm-start guess at the start of a solve (phi = the guess)
-    int stage;
-    int last;                  // the last pass the step's graph runs: a solve that needs another one stalls
+    int limit;                 // passes of a solve that a step's graph without refinement loops runs
+    int stalls, stage;         // such a graph: a solve that needs another pass stalls there
 };
 
 // A cavity whose refinement loop has ended (a batch runs passes while any cavity needs one) skips the pass.
@@ -946,9 +947,12 @@ __device__ void residual_body(const ResidualArgs& a, const Blk& k) {
             c->rel = sqrt(tot.v[0]) / c->rhs_norm;
             if (!isfinite(c->rel)) { c->error = kResidualNaN; set_loop(c, a.handle, a.use_handle, 0); return; }
             decide_loop(p, c, a.handle, a.use_handle);
-            if (a.last && c->cond && !c->error) {
-                c->stage = a.stage;
-                c->error = kStalled;
+            if (c->cond && !c->error && c->passes == a.limit) {
+                c->long_solves += 1;
+                if (a.stalls) {
+                    c->stage = a.stage;
+                    c->error = kStalled;
+                }
             }
         }
     }

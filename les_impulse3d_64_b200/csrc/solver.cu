@@ -243,12 +243,7 @@ public:
         check(cudaStreamSynchronize(stream_));
     }
     ~Solver() override {
-        for (int s = 0; s < 2; s++) {
-            if (exec_[s]) cudaGraphExecDestroy(exec_[s]);
-            if (graph_[s]) cudaGraphDestroy(graph_[s]);
-            if (texec_[s]) cudaGraphExecDestroy(texec_[s]);
-            if (tgraph_[s]) cudaGraphDestroy(tgraph_[s]);
-        }
+        drop_graphs();
         for (cudaEvent_t& e : kev_) if (e) cudaEventDestroy(e);
         if (stream_) cudaStreamSynchronize(stream_);
         arena_.release();
@@ -301,7 +296,7 @@ public:
     void queue_step(bool timing) {
         if (pending_.empty()) steps_before_ = hc_.steps;
         if (eager_) enqueue_step(par_, timing, true);
-        else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[par_], stream_));
+        else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[loops_][par_], stream_));
         pending_.push_back({par_});
         par_ ^= 1;
     }
@@ -327,14 +322,23 @@ public:
         }
         check(cudaGetLastError());
         probes_fresh_ = tail && !pending_copy.empty();
+        if (loops_) count_quiet_steps((int)queued);
         if (r) report(r);
+    }
+    // Graphs without the loops again once `patience_` steps in a row had no solve that needs them: 64 after the first
+    // stall, which costs about as much as the loops of so many steps, and twice as many after each further one.
+    void count_quiet_steps(int steps) {
+        quiet_ = hc_.long_solves == long_solves_ ? quiet_ + steps : 0;
+        long_solves_ = hc_.long_solves;
+        if (quiet_ >= patience_) loops_ = false;
     }
     // Wait for the queued steps and read the control block.  A step's graph runs one pressure pass per solve (two on the
     // tensor cores, whose FP32 transforms usually take a second): a conditional while-node for the rare further pass cost
     // 9 us per solve even when it ran nothing, the breaks in the chain of programmatic launches included (a step of
     // 32 x 32 x 8 cells 173 us with them, 146 without; 64^3 282 and 256).  A solve that needs more stalls: the rest of the
     // queued work returns at once, the state it reads being untouched, and the host finishes that step here, pass by pass.
-    // From then on the cavity's graphs have the while-nodes (loops_); the steps queued after it run through those.
+    // From then on the cavity steps through graphs with the while-nodes (loops_, see count_quiet_steps); the steps queued
+    // after it run through those.
     void settle() {
         if (batch_pending_) check(cudaDeviceSynchronize());       // they run on the batch's stream, which may be gone
         else check(cudaStreamSynchronize(stream_));
@@ -347,9 +351,10 @@ public:
         if (!pending_.empty()) settle();
     }
     void resume_stalled() {
-        stalls_++;
+        patience_ = stalls_++ ? std::min(2 * patience_, 1 << 14) : 64;
+        quiet_ = 0;
+        long_solves_ = hc_.long_solves;
         loops_ = true;
-        drop_graphs();
         tail_queued_ = false;
         const size_t stalled = (size_t)std::max(hc_.steps - steps_before_, 0LL);
         hc_.error = kOk;
@@ -363,7 +368,7 @@ public:
                 for (int s = stage + 1; s < 3; s++) enqueue_stage(q.par, s, false, true);
             } else {
                 ensure_graphs(false);
-                check(cudaGraphLaunch(exec_[q.par], stream_));
+                check(cudaGraphLaunch(exec_[1][q.par], stream_));
             }
             if (q.ring >= 0)
                 probes_kernel<T><<<1, 32, 0, stream_>>>(out_args(q.par ^ 1), probe_cells_, c_.n_probes,
@@ -698,7 +703,7 @@ public:
         for (int pass = 0; pass < (kms ? 2 : 1); pass++) {
             const bool timing = pass == 1;
             for (int i = 0; i < steps; i++) {
-                ensure_graphs(timing);                   // a step that stalls drops them
+                ensure_graphs(timing);                   // after a step that stalls, those with loops
                 if (flush) check(cudaMemsetAsync(flush_, i & 0xff, kFlushBytes, stream_));
                 const long long stalls = stalls_;
                 check(cudaEventRecord(ev.begin, stream_));
@@ -1167,10 +1172,11 @@ private:
         if (step_mode) launch_residual(st, praw_, h, use_h, 1);    // the residual of the guess
     }
     void launch_residual(cudaStream_t st, const double* phi, cudaGraphConditionalHandle h, int use_h, int start = 0,
-                         int last = 0, int stage = 0) {
+                         int stalls = 0, int stage = 0) {
         ResidualArgs a;
         a.start = start;
-        a.last = last;
+        a.limit = tc_fdm_ ? 2 : 1;
+        a.stalls = stalls;
         a.stage = stage;
         a.p = p_;
         for (int k = 0; k < 3; k++) { a.dw[k] = geo_.dw[k]; a.dinv_sp[k] = geo_.dinv_sp[k]; }
@@ -1191,11 +1197,10 @@ private:
     }
     // the passes of a step's graph without a loop: one, or two on the tensor cores, the last of which may stall the step
     void launch_passes(cudaStream_t st, double* phi, int stage) {
-        launch_transforms(st, phi, 0, 0);
-        launch_residual(st, phi, 0, 0, 0, !tc_fdm_, stage);
-        if (!tc_fdm_) return;
-        launch_transforms(st, phi, 0, 0);
-        launch_residual(st, phi, 0, 0, 0, 1, stage);
+        for (int pass = tc_fdm_ ? 2 : 1; pass > 0; pass--) {
+            launch_transforms(st, phi, 0, 0);
+            launch_residual(st, phi, 0, 0, 0, 1, stage);
+        }
     }
     // the six transforms of a pass (backend.cu:801-814)
     void launch_transforms(cudaStream_t st, double* phi, cudaGraphConditionalHandle h, int use_h) {
@@ -1366,23 +1371,26 @@ private:
         const char* env = std::getenv("CAVITY_GRAPHS");
         eager_ = env && env[0] == '0';
     }
-    // the step graphs of both state parities (timing: with events around the sweeps), captured on first use, so
-    // a solver that only takes part in batches or is only initialised never builds them
+    // the step graphs of both state parities, without or with refinement loops, or with events between the kernels
+    // (timing), captured on first use, so a solver that only takes part in batches or is only initialised never builds them
     void drop_graphs() {
+        auto drop = [](cudaGraph_t& g, cudaGraphExec_t& ex) {
+            if (ex) cudaGraphExecDestroy(ex);
+            if (g) cudaGraphDestroy(g);
+            ex = nullptr;
+            g = nullptr;
+        };
         for (int s = 0; s < 2; s++) {
-            if (exec_[s]) cudaGraphExecDestroy(exec_[s]);
-            if (graph_[s]) cudaGraphDestroy(graph_[s]);
-            if (texec_[s]) cudaGraphExecDestroy(texec_[s]);
-            if (tgraph_[s]) cudaGraphDestroy(tgraph_[s]);
-            exec_[s] = texec_[s] = nullptr;
-            graph_[s] = tgraph_[s] = nullptr;
+            drop(graph_[0][s], exec_[0][s]);
+            drop(graph_[1][s], exec_[1][s]);
+            drop(tgraph_[s], texec_[s]);
         }
     }
     void ensure_graphs(bool timing) {
         if (eager_) return;
         for (int S = 0; S < 2; S++) {
-            cudaGraph_t& g = timing ? tgraph_[S] : graph_[S];
-            cudaGraphExec_t& ex = timing ? texec_[S] : exec_[S];
+            cudaGraph_t& g = timing ? tgraph_[S] : graph_[loops_][S];
+            cudaGraphExec_t& ex = timing ? texec_[S] : exec_[loops_][S];
             if (ex) continue;
             check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
             enqueue_step(S, timing, false);
@@ -1512,6 +1520,8 @@ private:
     bool batch_pending_ = false;        // queued by a batch that has not waited for them
     bool loops_ = false;                // step graphs with conditional refinement loops (after a stalled solve)
     long long stalls_ = 0;              // stalled steps that the host finished
+    int patience_ = 0, quiet_ = 0;      // steps without a long solve until the loops go, and so far (count_quiet_steps)
+    int long_solves_ = 0;               // the control block's count when last looked at
     long long steps_before_ = 0;
     // fields: three buffer sets of velocity, impulse and potential (state, stage outputs)
     T* U_[3][3];
@@ -1535,8 +1545,8 @@ private:
     float *plane_, *fstage_, *probe_out_;
     int* probe_cells_;
     const double* centre_[3];
-    cudaGraph_t graph_[2] = {nullptr, nullptr}, tgraph_[2] = {nullptr, nullptr};
-    cudaGraphExec_t exec_[2] = {nullptr, nullptr}, texec_[2] = {nullptr, nullptr};
+    cudaGraph_t graph_[2][2] = {}, tgraph_[2] = {};              // graph_, exec_: [loops][state parity]
+    cudaGraphExec_t exec_[2][2] = {}, texec_[2] = {};
     // events of the timing graph: [kernel][stage][begin, end]; per-step means of the last time_steps call
     enum TimedKernel : int { kTkSweep = 0, kTkStart, kTkGuessResidual, kTkFinish, kTkTransforms, kNumTimed };
     cudaEvent_t kev_[2 * 3 * kNumTimed] = {};
