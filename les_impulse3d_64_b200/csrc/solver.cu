@@ -1589,6 +1589,28 @@ template <class T> class Batch : public BatchBase {
     using S_ = Solver<T>;
     static constexpr int kTY = S_::kTileTY, kTZ = S_::kTileTZ, kNT = S_::kTileNT;
 
+    // where one recorded launch's argument records sit in the argument buffer of a graph
+    struct LaunchSlot {
+        int kind, variant;
+        size_t smem, off, size;
+        dim3 grid;
+    };
+    struct Layout {
+        std::vector<LaunchSlot> launches;
+        size_t live = 0;                       // the slots' live flags (int each)
+    };
+
+    // One step graph of one state parity: its arguments, with their host copy, and the handles of its refinement loops.
+    struct StepGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        bool loops = false;
+        cudaGraphConditionalHandle handles[3] = {};
+        void* args = nullptr;
+        std::vector<unsigned char> host;
+        Layout layout;
+    };
+
 public:
     // `members` fill slots 0 .. n-1 of `capacity` slots; the other slots start empty (cavities of one size only)
     Batch(const std::vector<S_*>& members, int capacity) : m_(members) {
@@ -1627,7 +1649,6 @@ public:
             grids.resize(capacity, &f);           // empty slots take cavities of the first one's grid
             column_ = S_::column_height(grids, f.sms_);
         }
-        proto_ = m_[0];
         par_ = m_[0]->par_;
         nx_ = f.nx_;
         ny_ = f.ny_;
@@ -1655,18 +1676,15 @@ public:
         if (f.tc_fdm_) check(tc_transform_prepare_batched());
         if (f.tc_fdm_) check(tc_pair_prepare());
         check(pair_prepare());
-        for (const S_* s : m_) loops_ = loops_ || (s && s->loops_);
-        for (int S = 0; S < 2; S++) build(S);
-        proto_ = nullptr;        // members may leave and be destroyed from now on
+        ensure_graphs();
     }
     ~Batch() override {
         if (stream_) cudaStreamSynchronize(stream_);
         for (int S = 0; S < 2; S++) {
-            if (exec_[S]) cudaGraphExecDestroy(exec_[S]);
-            if (graph_[S]) cudaGraphDestroy(graph_[S]);
-            if (dargs_[S]) cudaFree(dargs_[S]);
+            drop(plain_[S]);
+            drop(looping_[S]);
+            drop(timing_[S]);
         }
-        drop_timing();
         for (cudaEvent_t& e : tev_)
             if (e) cudaEventDestroy(e);
         if (stream_) cudaStreamDestroy(stream_);
@@ -1675,14 +1693,8 @@ public:
     int size() const override { return (int)m_.size(); }
 
     void step_async(int count) override {
-        if (!queued_ && !loops_) {       // a member's solve stalled (Solver::settle): graphs with refinement loops from now on
-            for (S_* s : m_)
-                if (s && s->loops_) {
-                    rebuild_with_loops(s);
-                    break;
-                }
-        }
-        for (int i = 0; i < count; i++) launch_step(exec_);
+        StepGraph* g = ensure_graphs();
+        for (int i = 0; i < count; i++) launch_step(g);
     }
     // Per-step device time (ms, summed over the three stages) of the batch's parts: the sweeps, the projection
     // starts with the residuals of their guesses, the first pressure pass of each stage (transforms and
@@ -1693,25 +1705,11 @@ public:
         if (queued_) fail("batch: steps are queued; sync first");
         if (!tev_[0])
             for (cudaEvent_t& e : tev_) check(cudaEventCreate(&e));
-        for (S_* s : m_)
-            if (s && !proto_) proto_ = s;                 // what the empty slots record
-        if (!proto_) fail("batch part times: every slot is empty");
-        drop_timing();
-        {
-            struct Restore {
-                Batch* b;
-                const bool loops;
-                ~Restore() {
-                    b->loops_ = loops;
-                    b->proto_ = nullptr;
-                }
-            } restore{this, loops_};
-            loops_ = true;
-            for (int S = 0; S < 2; S++) build(S, true);
-        }
+        if (!first_member()) fail("batch part times: every slot is empty");
+        for (int S = 0; S < 2; S++) build(timing_[S], S, true, true);
         for (int k = 0; k < kParts; k++) ms[k] = 0;
         for (int i = 0; i < steps; i++) {
-            launch_step(texec_);
+            launch_step(timing_);
             sync(nullptr);
             for (int stage = 0; stage < 3; stage++)
                 for (int k = 0; k < kParts; k++) {
@@ -1724,22 +1722,34 @@ public:
     static constexpr int kParts = 4;
 
 private:
-    void drop_timing() {
-        for (int S = 0; S < 2; S++) {
-            if (texec_[S]) cudaGraphExecDestroy(texec_[S]);
-            if (tgraph_[S]) cudaGraphDestroy(tgraph_[S]);
-            if (targs_[S]) cudaFree(targs_[S]);
-            texec_[S] = nullptr;
-            tgraph_[S] = nullptr;
-            targs_[S] = nullptr;
-        }
+    static void drop(StepGraph& g) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (g.graph) cudaGraphDestroy(g.graph);
+        if (g.args) cudaFree(g.args);
+        g = StepGraph();
     }
-    void launch_step(cudaGraphExec_t* exec) {
+    S_* first_member() const {
+        for (S_* s : m_)
+            if (s) return s;
+        return nullptr;
+    }
+    // the graphs (of both parities) the next steps run: with refinement loops while a member's own have them
+    // (Solver::settle), without otherwise; each is built when first needed
+    StepGraph* ensure_graphs() {
+        bool loops = false;
+        for (const S_* s : m_) loops = loops || (s && s->loops_);
+        StepGraph* g = loops ? looping_ : plain_;
+        if (!first_member()) return plain_[0].exec ? plain_ : looping_;      // only empty slots: whichever there is
+        for (int S = 0; S < 2; S++)
+            if (!g[S].exec) build(g[S], S, loops);
+        return g;
+    }
+    void launch_step(StepGraph* g) {
         {
             for (size_t k = 0; k < m_.size(); k++)
                 if (m_[k] && m_[k]->par_ != (par_ ^ d_[k]))
                     fail("batch: the cavities' states have diverged (a failed step); rebuild the batch");
-            check(cudaGraphLaunch(exec[par_], stream_));
+            check(cudaGraphLaunch(g[par_].exec, stream_));
             for (S_* s : m_) {
                 if (!s) continue;
                 if (s->pending_.empty()) s->steps_before_ = s->hc_.steps;
@@ -1795,29 +1805,33 @@ public:
             if (s->nx_ != nx_ || s->ny_ != ny_ || s->nz_ != nz_) fail("batch: the cavity's grid size differs from the batch's");
             if (s->tc_fdm_ != tc_fdm_ || s->sweep_kind_ != sweep_kind_) fail("batch: the cavity's kernels differ from the batch's");
             d_[slot] = s->par_ ^ par_;
-            for (int S = 0; S < 2; S++) {
-                std::vector<LaunchRecord> rec;
-                {
-                    RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_, column_);
-                    record_member(*s, S ^ d_[slot], S);
+            for (int S = 0; S < 2; S++)
+                for (StepGraph* g : {&plain_[S], &looping_[S]}) {
+                    if (!g->exec) continue;
+                    std::vector<LaunchRecord> rec;
+                    {
+                        RecordGuard guard(&rec, (int)m_.size(), dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_, column_);
+                        record_member(*s, S ^ d_[slot], *g);
+                    }
+                    const Layout& L = g->layout;
+                    if (rec.size() != L.launches.size()) fail("batch: the cavity's launch sequence differs from the batch's");
+                    for (size_t j = 0; j < rec.size(); j++) {
+                        const LaunchSlot& ls = L.launches[j];
+                        if (rec[j].kind != ls.kind || rec[j].variant != ls.variant || rec[j].smem != ls.smem ||
+                            rec[j].args.size() != ls.size || rec[j].grid.x != ls.grid.x || rec[j].grid.y != ls.grid.y ||
+                            rec[j].grid.z != ls.grid.z)
+                            fail("batch: the cavity's launch sequence differs from the batch's");
+                        std::memcpy(g->host.data() + ls.off + (size_t)slot * ls.size, rec[j].args.data(), ls.size);
+                    }
                 }
-                const Layout& L = layout_[S];
-                if (rec.size() != L.launches.size()) fail("batch: the cavity's launch sequence differs from the batch's");
-                for (size_t j = 0; j < rec.size(); j++) {
-                    const LaunchSlot& ls = L.launches[j];
-                    if (rec[j].kind != ls.kind || rec[j].variant != ls.variant || rec[j].smem != ls.smem ||
-                        rec[j].args.size() != ls.size || rec[j].grid.x != ls.grid.x || rec[j].grid.y != ls.grid.y ||
-                        rec[j].grid.z != ls.grid.z)
-                        fail("batch: the cavity's launch sequence differs from the batch's");
-                    std::memcpy(host_[S].data() + ls.off + (size_t)slot * ls.size, rec[j].args.data(), ls.size);
-                }
-            }
         }
         m_[slot] = s;
-        for (int S = 0; S < 2; S++) {
-            reinterpret_cast<int*>(host_[S].data() + layout_[S].live)[slot] = s ? 1 : 0;
-            check(cudaMemcpyAsync(dargs_[S], host_[S].data(), host_[S].size(), cudaMemcpyHostToDevice, stream_));
-        }
+        for (int S = 0; S < 2; S++)
+            for (StepGraph* g : {&plain_[S], &looping_[S]}) {
+                if (!g->exec) continue;
+                reinterpret_cast<int*>(g->host.data() + g->layout.live)[slot] = s ? 1 : 0;
+                check(cudaMemcpyAsync(g->args, g->host.data(), g->host.size(), cudaMemcpyHostToDevice, stream_));
+            }
         check(cudaStreamSynchronize(stream_));
     }
 
@@ -1853,57 +1867,48 @@ private:
         if (!s->pending_.empty()) fail("batch: a cavity has queued steps; sync it first");
     }
 
-    // where one recorded launch's argument records sit in the argument buffer of a graph
-    struct LaunchSlot {
-        int kind, variant;
-        size_t smem, off, size;
-        dim3 grid;
-    };
-    struct Layout {
-        std::vector<LaunchSlot> launches;
-        size_t live = 0;                       // the slots' live flags (int each)
-    };
-
-    // The launches of one cavity's step, for the cavity's state parity Sm inside the graph of batch parity S
-    // (whose while-node handles the loop kernels set), in the order the graph runs them.  `part` selects one
-    // piece of the sequence (see sequence); -1 all of them.
-    void member_part(S_& s, int Sm, int S, int stage, int part) {
+    // The launches of one cavity's step, for the cavity's state parity Sm inside the graph `g` (whose while-node handles
+    // the loop kernels set), in the order the graph runs them.  `part` selects one piece of the sequence (see sequence).
+    void member_part(S_& s, int Sm, const StepGraph& g, int stage, int part) {
         const int Xs = Sm ^ 1, Ys = 2;
         const int in = stage == 0 ? Sm : stage == 1 ? Xs : Ys;
         const int out = stage == 1 ? Ys : Xs;
         const int cur = stage == 1 ? Xs : Ys;
-        const cudaGraphConditionalHandle h = loops_ ? handles_[S][stage] : 0;
+        const cudaGraphConditionalHandle h = g.handles[stage];
         cudaStream_t st = part == 3 ? body_stream_ : stream_;
         switch (part) {
         case 0: s.launch_momentum(st, stage, Sm, in, out); break;
-        case 1: s.launch_start(st, s.M_[out], true, stage, Sm, cur, h, loops_ ? 2 : 0); break;
+        case 1: s.launch_start(st, s.M_[out], true, stage, Sm, cur, h, g.loops ? 2 : 0); break;
         case 2:
-            if (!loops_) {
+            if (!g.loops) {
                 s.launch_passes(st, s.praw_, stage);
                 break;
             }
         case 3:
-            if (loops_) s.launch_pass(st, s.praw_, h, 2);
+            if (g.loops) s.launch_pass(st, s.praw_, h, 2);
             break;
         case 4: s.launch_finish(st, s.M_[out], s.U_[out], s.PHI_[out], true, stage, stage == 2); break;
         }
     }
-    void record_member(S_& s, int Sm, int S) {
+    void record_member(S_& s, int Sm, const StepGraph& g) {
         s.launch_step_begin(stream_);
         for (int stage = 0; stage < 3; stage++)
-            for (int part = 0; part < 5; part++) member_part(s, Sm, S, stage, part);
+            for (int part = 0; part < 5; part++) member_part(s, Sm, g, stage, part);
     }
 
     // run `fn(member, slot)` on every slot (an empty slot records the first member: its records are never read,
-    // the slot being dead) with a recorder installed, append the argument records of each recorded launch to
-    // `host` (one contiguous array per launch, slot after slot) and, when `launch`, issue the batched launches
-    template <class F> void emit(cudaStream_t st, F fn, std::vector<unsigned char>& host, Layout& L, bool launch) {
+    // the slot being dead) with a recorder installed, append the argument records of each recorded launch to the
+    // graph's host copy (one contiguous array per launch, slot after slot) and, when `launch`, issue the batched launches
+    template <class F> void emit(cudaStream_t st, F fn, StepGraph& g, bool launch) {
+        std::vector<unsigned char>& host = g.host;
+        Layout& L = g.layout;
         const size_t B = m_.size();
+        S_* const stand_in = first_member();
         std::vector<std::vector<LaunchRecord>> recs(B);
         for (size_t b = 0; b < B; b++) {
             RecordGuard guard(&recs[b], (int)B, dgemm_tile_, pairs_, tc_pairs_, fused_start_, wide_, column_);
             if (m_[b]) fn(*m_[b], (int)b);
-            else fn(*proto_, 0);
+            else fn(*stand_in, 0);
         }
         for (size_t b = 1; b < B; b++) {
             bool same = recs[b].size() == recs[0].size();
@@ -1913,7 +1918,7 @@ private:
             }
             if (!same) fail("batch: the cavities' launch sequences differ");
         }
-        const unsigned char* dbase = static_cast<const unsigned char*>(dargs_cur_);
+        const unsigned char* dbase = static_cast<const unsigned char*>(g.args);
         for (size_t j = 0; j < recs[0].size(); j++) {
             const size_t sz = recs[0][j].args.size();
             const size_t off = align256(host.size());
@@ -2002,137 +2007,88 @@ private:
     // the step of batch parity S (as Solver::enqueue_step, each slot at its own state parity S ^ d); `launch` =
     // false only records (sizes the argument buffer), true captures the batched launches into the graph being
     // built on stream_
-    void sequence(int S, std::vector<unsigned char>& host, Layout& L, bool launch, bool timing = false) {
+    void sequence(StepGraph& g, int S, bool launch, bool timing) {
         // timing: events before and after the parts of each stage outside the refinement loop (part_times)
         auto mark = [&](int stage, int part, int end) {
             if (timing && launch)
                 check(cudaEventRecordWithFlags(tev_[(stage * kParts + part) * 2 + end], stream_, cudaEventRecordExternal));
         };
-        L.live = 0;
-        host.resize(align256(sizeof(int) * m_.size()));
-        for (size_t i = 0; i < m_.size(); i++) reinterpret_cast<int*>(host.data())[i] = m_[i] ? 1 : 0;
+        g.host.assign(align256(sizeof(int) * m_.size()), 0);
+        g.layout = Layout();
+        item_lists_.clear();
+        for (size_t i = 0; i < m_.size(); i++) reinterpret_cast<int*>(g.host.data())[i] = m_[i] ? 1 : 0;
         auto par = [&](int b) { return S ^ d_[b]; };
-        emit(stream_, [&](S_& s, int) { s.launch_step_begin(stream_); }, host, L, launch);
+        emit(stream_, [&](S_& s, int) { s.launch_step_begin(stream_); }, g, launch);
         for (int stage = 0; stage < 3; stage++) {
             mark(stage, 0, 0);
-            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 0); }, host, L, launch);
+            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 0); }, g, launch);
             mark(stage, 0, 1);
-            cudaGraph_t g = nullptr;
+            cudaGraph_t graph = nullptr;
             const cudaGraphNode_t* deps = nullptr;
             size_t ndeps = 0;
             cudaStreamCaptureStatus status;
-            if (launch && loops_) {
-                check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &g, &deps, &ndeps));
-                check(cudaGraphConditionalHandleCreate(&handles_[S][stage], g, 0, cudaGraphCondAssignDefault));
+            if (launch && g.loops) {
+                check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &graph, &deps, &ndeps));
+                check(cudaGraphConditionalHandleCreate(&g.handles[stage], graph, 0, cudaGraphCondAssignDefault));
             }
             mark(stage, 1, 0);
-            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 1); }, host, L, launch);
+            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 1); }, g, launch);
             mark(stage, 1, 1);
             // the first pass outside the loop (see Solver::captured_loop), then the loop
             mark(stage, 2, 0);
-            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 2); }, host, L, launch);
+            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 2); }, g, launch);
             mark(stage, 2, 1);
-            if (!loops_) {
+            if (!g.loops) {
                 // the passes are all in the chain
             } else if (launch) {
-                check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &g, &deps, &ndeps));
+                check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, &graph, &deps, &ndeps));
                 cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
                 cp.type = cudaGraphNodeTypeConditional;
-                cp.conditional.handle = handles_[S][stage];
+                cp.conditional.handle = g.handles[stage];
                 cp.conditional.type = cudaGraphCondTypeWhile;
                 cp.conditional.size = 1;
                 cudaGraphNode_t node;
-                check(cudaGraphAddNode(&node, g, deps, ndeps, &cp));
+                check(cudaGraphAddNode(&node, graph, deps, ndeps, &cp));
                 cudaGraph_t body = cp.conditional.phGraph_out[0];
                 check(cudaStreamBeginCaptureToGraph(body_stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-                emit(body_stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 3); }, host, L, launch);
+                emit(body_stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 3); }, g, launch);
                 check(cudaStreamEndCapture(body_stream_, &body));
                 check(cudaStreamUpdateCaptureDependencies(stream_, &node, 1, cudaStreamSetCaptureDependencies));
             } else {
-                emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 3); }, host, L, launch);
+                emit(stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 3); }, g, launch);
             }
             mark(stage, 3, 0);
-            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), S, stage, 4); }, host, L, launch);
+            emit(stream_, [&](S_& s, int b) { member_part(s, par(b), g, stage, 4); }, g, launch);
             mark(stage, 3, 1);
         }
     }
-    // the plain graphs again, with refinement loops; empty slots record `proto`
-    void rebuild_with_loops(S_* proto) {
-        loops_ = true;
-        proto_ = proto;
-        for (int S = 0; S < 2; S++) {
-            check(cudaGraphExecDestroy(exec_[S]));
-            check(cudaGraphDestroy(graph_[S]));
-            check(cudaFree(dargs_[S]));
-            exec_[S] = nullptr;
-            graph_[S] = nullptr;
-            dargs_[S] = nullptr;
-            build(S);
-        }
-        proto_ = nullptr;
-    }
-    // the step graph of batch parity S; with `timing` the instrumented twin (part_times), built from the current
-    // members with its own argument buffer and refinement-loop handles (the plain graph's are kept)
-    void build(int S, bool timing = false) {
-        if (timing) {
-            cudaGraphConditionalHandle saved[3] = {handles_[S][0], handles_[S][1], handles_[S][2]};
-            std::vector<unsigned char> host;
-            Layout L;
-            item_lists_.clear();
-            sequence(S, host, L, false);
-            check(cudaMalloc(&targs_[S], std::max<size_t>(host.size(), 256)));
-            dargs_cur_ = targs_[S];
-            host.clear();
-            item_lists_.clear();
-            L = Layout();
-            check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            sequence(S, host, L, true, true);
-            check(cudaStreamEndCapture(stream_, &tgraph_[S]));
-            check(cudaGraphInstantiate(&texec_[S], tgraph_[S], 0));
-            check(cudaMemcpy(targs_[S], host.data(), host.size(), cudaMemcpyHostToDevice));
-            for (int k = 0; k < 3; k++) handles_[S][k] = saved[k];
-            dargs_cur_ = dargs_[S];
-            return;
-        }
-        std::vector<unsigned char> host;
-        Layout L;
-        item_lists_.clear();
-        sequence(S, host, L, false);
-        check(cudaMalloc(&dargs_[S], std::max<size_t>(host.size(), 256)));
-        dargs_cur_ = dargs_[S];
-        host.clear();
-        item_lists_.clear();
-        layout_[S] = Layout();
+    // build the step graph of batch parity S from the current members; with `timing` events between the parts
+    // (part_times).  The first pass over the sequence sizes the argument buffer, the second captures.
+    void build(StepGraph& g, int S, bool loops, bool timing = false) {
+        drop(g);
+        g.loops = loops;
+        sequence(g, S, false, timing);
+        check(cudaMalloc(&g.args, std::max<size_t>(g.host.size(), 256)));
         check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        sequence(S, host, layout_[S], true);
-        check(cudaStreamEndCapture(stream_, &graph_[S]));
-        check(cudaGraphInstantiate(&exec_[S], graph_[S], 0));
-        check(cudaMemcpy(dargs_[S], host.data(), host.size(), cudaMemcpyHostToDevice));
-        host_[S] = std::move(host);
+        sequence(g, S, true, timing);
+        check(cudaStreamEndCapture(stream_, &g.graph));
+        check(cudaMemcpy(g.args, g.host.data(), g.host.size(), cudaMemcpyHostToDevice));
+        check(cudaGraphInstantiate(&g.exec, g.graph, 0));
     }
 
     std::vector<S_*> m_;                      // slot -> cavity (nullptr: empty)
     std::vector<int> d_;                      // slot -> its cavity's state parity relative to the batch's
-    S_* proto_ = nullptr;                     // a member, while the graphs are built
     int par_ = 0;                             // the batch's state parity: the graph the next step launches
     bool queued_ = false;
     int nx_ = 0, ny_ = 0, nz_ = 0, sweep_kind_ = 0;
     bool tc_fdm_ = false;
     cudaStream_t stream_ = nullptr, body_stream_ = nullptr;
-    cudaGraph_t graph_[2] = {nullptr, nullptr}, tgraph_[2] = {nullptr, nullptr};
-    cudaGraphExec_t exec_[2] = {nullptr, nullptr}, texec_[2] = {nullptr, nullptr};
+    StepGraph plain_[2], looping_[2], timing_[2];      // by state parity: without and with refinement loops; part_times
     cudaEvent_t tev_[3 * kParts * 2] = {};
-    void* targs_[2] = {nullptr, nullptr};     // argument buffers of the timing graphs
-    cudaGraphConditionalHandle handles_[2][3] = {};
-    void* dargs_[2] = {nullptr, nullptr};
-    void* dargs_cur_ = nullptr;
-    std::vector<unsigned char> host_[2];      // host copies of the argument buffers
-    Layout layout_[2];
     bool mixed_sizes_ = false;
     int column_ = 0;            // half the height of the column walk's chunks (g_batch_column)
     int wide_ = 0;              // the phases of the paired pass that run the streamed kernel (g_batch_wide)
     int pairs_ = 0;             // FP64 passes as paired launches (every member's axes at most 128 cells)
-    bool loops_ = false;        // conditional refinement loops in the graphs
     bool fused_start_ = false;  // projection starts with their guesses' residuals in one launch
     int tc_pairs_ = 0;          // tensor-core passes as paired launches (g_batch_tc_pairs)
     int dgemm_tile_ = 0;

@@ -2,6 +2,8 @@
 each leaves the cavity where the same steps leave one that runs kernel by kernel (CAVITY_GRAPHS=0), whose refinement loop
 the host drives anyway.  Two forms stall in their first step: the tensor-core transforms (two passes a solve) above 2^18
 cells, where the projection starts in two launches, and the FP64 ones (one pass) in one launch."""
+import time
+
 import numpy as np
 import pytest
 
@@ -203,3 +205,47 @@ def test_graphs_without_loops_return(monkeypatch):
         finally:
             cav.close()
     assert fastest[3e-15] < 1.12 * fastest[1e-9], fastest
+
+
+def test_batch_follows_its_members(monkeypatch):
+    """A batch runs graphs with refinement loops while it holds a cavity that stalled, and others once that one has left its
+    slot: then its steps take as long as a batch's that never held it, and the other member's are the same throughout."""
+    monkeypatch.setenv('CAVITY_FDM', '')
+
+    def cavity(rtol, seed):
+        cav = Cavity(workloads.settings(32, 400.0, nz=8, beta=1.5, cfl=0.5, fdm_rtol=rtol))
+        cav.initialize(*workloads.initial_noise(cav.shapes, 1e-2, seed))
+        return cav
+
+    def seconds(batch):
+        t = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            batch.step_async(40)
+            batch.sync()
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    stalls, member, alone = cavity(3e-15, 5), cavity(1e-9, 6), cavity(1e-9, 6)
+    batch, calm = Batch([stalls, member]), Batch([alone], capacity=2)
+    try:
+        before = stalls.pressure_passes()
+        for b in (batch, calm):
+            for _ in range(2):
+                b.step_async(1)
+                b.sync()
+        assert stalls.pressure_passes() - before > 2 * 3
+        batch.set_member(0, None)
+        after, never = seconds(batch), seconds(calm)
+        batch.set_member(0, stalls)
+        for b in (batch, calm):
+            b.step_async(2)
+            b.sync()
+        assert_same(member, alone)
+        assert stalls.report()['steps'] == 4
+        assert after < 1.12 * never
+    finally:
+        batch.close()
+        calm.close()
+        for cav in (stalls, member, alone):
+            cav.close()
