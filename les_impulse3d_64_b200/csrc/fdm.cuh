@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <vector>
 
 #include "kernels.cuh"
 
@@ -730,6 +731,25 @@ inline bool pair_pass_fits(int nx, int ny, int nz) {
 inline bool pair_wide(int phase, int nx, int ny, int nz) {
     if (g_launch_record) return (g_batch_wide >> phase) & 1;
     return phase == kPairZ ? nz > kPairMax : nx > kPairMax || ny > kPairMax;
+}
+// Whether a batch of these grids, all of them within pair_pass_fits, runs its passes as three paired launches.  A member of
+// up to 64 cells an axis beside a longer one runs the streamed kernel too, on 128-row tiles: that costs more than the three
+// launches save once many members of 33 to 64 cells share it.  Measured, mixed form, us per step, three and six launches:
+// 8, 12 and 24 of 64^3 with one of 66^3 1330 and 1373, 1772 and 1729, 3226 and 3008; 16 of 64^3 with four of 96^3 3869 and
+// 3886, 24 with two 3758 and 3632; 24 and 48 of 48^3 with one of 72^3 2197 and 2184, 2991 and 2926; 96 of 32^3 with one of
+// 66^3 1909 and 2107.  Where only the z phase is streamed three are faster (24 of 64^3 with 8 x 8 x 66: 2636 and 2791).
+struct PairGrid { int nx, ny, nz; };
+inline bool pair_batch_pays(const std::vector<PairGrid>& grids) {
+    long long streamed = 0, narrow = 0;
+    bool plane = false;
+    for (const PairGrid& g : grids) {
+        const long long cells = (long long)g.nx * g.ny * g.nz;
+        const bool xy = g.nx > kPairMax || g.ny > kPairMax;
+        plane = plane || xy;
+        if (xy || g.nz > kPairMax) streamed += cells;
+        else if (std::max(g.nx, g.ny) > 32) narrow += cells;
+    }
+    return !plane || narrow <= (1LL << 21) + streamed;
 }
 inline int current_sm_count() {
     int dev = 0, sms = 148;

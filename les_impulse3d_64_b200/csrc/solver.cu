@@ -1630,13 +1630,17 @@ public:
         // cavities of different sizes share one FP64 transform tile: the large one when all of them together
         // have two 64 x 64 tiles per SM in the largest transform
         if (mixed_sizes_) dgemm_tile_ = tiles64 >= 2 * f.sms_ ? 64 : 32;
-        // FP64 passes as paired launches when every member's axes allow them (and CAVITY_FDM_FUSED names no
-        // other form), a phase by the streamed kernel when any member needs it
+        // FP64 passes as paired launches when every member's axes allow them and they are the faster (or CAVITY_FDM_FUSED
+        // names the form), a phase by the streamed kernel when any member needs it
         {
             bool fits = true;
-            for (const S_* s : m_) fits = fits && pair_pass_fits(s->nx_, s->ny_, s->nz_);
+            std::vector<PairGrid> sizes;
+            for (const S_* s : m_) {
+                fits = fits && pair_pass_fits(s->nx_, s->ny_, s->nz_);
+                sizes.push_back({s->nx_, s->ny_, s->nz_});
+            }
             const int e = pass_form_from_env();
-            pairs_ = fits && (e < 0 || e == kPassPairs) ? 1 : 0;
+            pairs_ = fits && (e < 0 ? pair_batch_pays(sizes) : e == kPassPairs) ? 1 : 0;
             for (const S_* s : m_)
                 for (int ph = 0; ph < 3; ph++) wide_ |= pair_wide(ph, s->nx_, s->ny_, s->nz_) << ph;
             bool tc_fits = true;
