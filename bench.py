@@ -163,10 +163,12 @@ def profile_traffic(workload):
     return None
 
 
-def sweep_kernel_name(precision, settings=None):
-    """The momentum-sweep kernel the library runs: the shared-memory tile kernel in the FP64 form, and in the mixed form
-    its packed two-cells-per-thread variant or, for the named workloads of 2^19 cells and more, the walk up columns,
-    unless CAVITY_SWEEP selects another."""
+def sweep_kernel_name(precision, cav=None):
+    """The momentum-sweep kernel of the steps of `cav`; without one, the tile kernel that a precision form starts from:
+    one cell per thread in the FP64 form, two in packed arithmetic in the mixed form, unless CAVITY_SWEEP selects
+    another."""
+    if cav is not None:
+        return cav.sweep_kernel()
     kind = os.environ.get('CAVITY_SWEEP', '')
     if kind == 'face':
         return 'momentum_kernel'
@@ -174,8 +176,6 @@ def sweep_kernel_name(precision, settings=None):
         return 'sweep_march_kernel'
     if kind == 'tile' or precision == 'fp64':
         return 'sweep_tile_kernel'
-    if settings and settings['nx'] * settings['ny'] * settings['nz'] >= 1 << 19 and os.environ.get('CAVITY_COLUMN') != '0':
-        return 'sweep_column_kernel'
     return 'sweep_pair_kernel'
 
 
@@ -376,6 +376,7 @@ def run_ours(args, ranks):
     ktimes = cav.kernel_times()
     passes = cav.pressure_passes() - passes0
     device_bytes = cav.device_bytes()
+    sweep = sweep_kernel_name(precision, cav)
     per_pass = (cav.kernels_per_step(1) - cav.kernels_per_step(0)) // 3       # transforms + residual
     launches = args.steps * cav.kernels_per_step(0) + per_pass * passes_in_timed(passes, args, cav)
     cav.close()
@@ -451,7 +452,7 @@ def run_ours(args, ranks):
                                'h2d_bytes_per_step': h2d, 'd2h_bytes_per_step': d2h},
         'gpu_launches': launches,
         'pressure_passes_per_stage': passes / (3 * (2 * args.steps + args.warmup)) if args.steps else None,
-        'roofline': {'kernel': sweep_kernel_name(precision, s), 'bound': 'hbm', 'achieved': achieved, 'peak': peak,
+        'roofline': {'kernel': sweep, 'bound': 'hbm', 'achieved': achieved, 'peak': peak,
                      'peak_kind': peak_kind, 'unit': 'GB/s', 'frac': achieved / peak,
                      'traffic': profile_traffic(args.workload), 'ms_per_launch': kernel_s * 1e3},
         'stencil_kernels': cell_kernels,

@@ -133,6 +133,8 @@ CavitySolver* cavity_default(void);
 /* Number of kernels one step launches (fixed part plus per pressure pass, for the cavity's transform launches) for
  * the counts it reports. */
 int cavity_kernels_per_step(const CavitySolver* s, int phi_passes_per_stage);
+/* Name of the momentum-sweep kernel that this cavity's own steps launch (NULL for an invalid handle). */
+const char* cavity_sweep_kernel(const CavitySolver* s);
 /* Queued steps with per-step outputs (no counterpart in the reference, whose run script makes a blocking
  * round trip per step for solver_probes and solver_add_statistics): queue `count` steps, each followed on the
  * device by its probe values (into a library-owned ring of pinned host memory, at most 4096 steps between

@@ -305,6 +305,12 @@ class Cavity:
     def kernels_per_step(self, passes_per_stage):
         return int(self.lib.cavity_kernels_per_step(self.handle, int(passes_per_stage)))
 
+    def sweep_kernel(self):
+        """Name of the momentum-sweep kernel this cavity's own steps launch."""
+        self.lib.cavity_sweep_kernel.argtypes = [ct.c_void_p]
+        self.lib.cavity_sweep_kernel.restype = ct.c_char_p
+        return self.lib.cavity_sweep_kernel(self.handle).decode()
+
     def pressure_passes(self):
         return int(self.lib.cavity_pressure_passes(self.handle))
 

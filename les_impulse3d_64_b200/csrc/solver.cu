@@ -177,6 +177,7 @@ public:
     virtual void time_steps(int warmup, int steps, int flush, float* ms, float* kms) = 0;
     virtual void kernel_times(double* ms) const = 0;
     virtual int kernels_per_step(int passes) const = 0;
+    virtual const char* sweep_kernel() const = 0;
     virtual long long pressure_passes() const = 0;
     virtual void autotune(int steps, int* chunks, int* dgemm_tile, int* fused, float* ms) = 0;
     void step(CavityReport* r) {
@@ -685,6 +686,12 @@ public:
         if (tc_fdm_) return tc_pair_used(nx_, ny_, nz_) ? 3 : 6;
         const int f = pass_form(fdm_, form_env_ >= 0 ? form_env_ : tune_.fused);
         return f == kPassPairs ? 3 : f == kPassOneLaunch ? 1 : 6;
+    }
+    const char* sweep_kernel() const override {
+        if (sweep_kind_ == kSweepFace) return "momentum_kernel";
+        if (sweep_kind_ == kSweepMarch) return "sweep_march_kernel";
+        if (sweep_kind_ == kSweepTile) return "sweep_tile_kernel";
+        return column_height() ? "sweep_column_kernel" : "sweep_pair_kernel";
     }
     long long pressure_passes() const override { return hc_.pass_count; }
 
@@ -2406,6 +2413,7 @@ int cavity_checkpoint_load(CavitySolver* s, const void* src, int src_is_device) 
     });
 }
 int cavity_kernels_per_step(const CavitySolver* s, int passes) { return s && s->s ? s->s->kernels_per_step(passes) : -1; }
+const char* cavity_sweep_kernel(const CavitySolver* s) { return s && s->s ? s->s->sweep_kernel() : nullptr; }
 int cavity_fdm_pass(int nx, int ny, int nz, const double* const s[3], const double* const st[3],
                     const double* inv_lambda, const double* r, double* phi, void* stream) {
     return safely([&] { cavity::fdm_pass(nx, ny, nz, s, st, inv_lambda, r, phi, (cudaStream_t)stream); });
