@@ -42,6 +42,39 @@ def assert_same(a, b):
 
 
 @pytest.mark.parametrize('form', FORMS)
+def test_queued_outputs(form, monkeypatch):
+    """Steps queued with their outputs, the first of which stalls, and a batch's: the same state, probes, statistics and
+    passes as step by step (the batch's fields to 1e-6: its sums group their terms by other blocks)."""
+    queued, member, eager = (make(form, monkeypatch, eager=e) for e in (False, False, True))
+    batch = Batch([member])
+    try:
+        queued.step_outputs_async(4, statistics=True)
+        report, values = queued.sync_outputs()
+        batch.step_async(4)
+        batched = batch.sync()[0]
+        stalling_step(eager, form)
+        eager.add_statistics(eager.report()['dt'])
+        passes, probes = [eager.report()['phi_passes']], [eager.probes()]
+        for _ in range(3):
+            passes.append(eager.step()['phi_passes'])
+            probes.append(eager.probes())
+            eager.add_statistics(eager.report()['dt'])
+        assert form != 'tc' or passes[0] > 2              # more than its graph runs
+        assert report == eager.report() and batched['steps'] == 4
+        assert queued.pressure_passes() == eager.pressure_passes()
+        assert np.array_equal(values, np.array(probes))
+        assert np.array_equal(queued.statistics(), eager.statistics())
+        assert_same(queued, eager)
+        for k in FIELDS:
+            x, y = member.field(k), eager.field(k)
+            assert np.abs(x - y).max() <= 1e-6 * np.abs(y).max(), k
+    finally:
+        batch.close()
+        for cav in (queued, member, eager):
+            cav.close()
+
+
+@pytest.mark.parametrize('form', FORMS)
 def test_time_steps(form, monkeypatch):
     """The first timed step stalls: the steps go on, and its time runs to the end of the host's part."""
     timed, eager = make(form, monkeypatch), make(form, monkeypatch, eager=True)
