@@ -152,14 +152,14 @@ def measured_peaks():
     return 6650.0, 'fallback'
 
 
-def profile_traffic(workload):
-    """DRAM bytes per momentum-sweep launch from the committed ncu summary (None if absent)."""
-    p = ROOT / 'profiles' / f'momentum_sweep_{workload}.md'
-    if not p.is_file():
-        return None
-    for line in p.read_text().splitlines():
-        if line.startswith('traffic_bytes_per_launch:'):
-            return float(line.split(':', 1)[1])
+def profile_traffic(workload, kernel):
+    """DRAM bytes per launch of the momentum sweep `kernel` from the committed ncu summary of it (None if absent)."""
+    for p in sorted((ROOT / 'profiles').glob(f'momentum_sweep_*{workload}.md')):
+        title, *lines = p.read_text().splitlines()
+        if kernel in title:
+            for line in lines:
+                if line.startswith('traffic_bytes_per_launch:'):
+                    return float(line.split(':', 1)[1])
     return None
 
 
@@ -454,7 +454,7 @@ def run_ours(args, ranks):
         'pressure_passes_per_stage': passes / (3 * (2 * args.steps + args.warmup)) if args.steps else None,
         'roofline': {'kernel': sweep, 'bound': 'hbm', 'achieved': achieved, 'peak': peak,
                      'peak_kind': peak_kind, 'unit': 'GB/s', 'frac': achieved / peak,
-                     'traffic': profile_traffic(args.workload), 'ms_per_launch': kernel_s * 1e3},
+                     'traffic': profile_traffic(args.workload, sweep), 'ms_per_launch': kernel_s * 1e3},
         'stencil_kernels': cell_kernels,
         'transforms': transforms_roofline(s, ranks.max(ktimes['transforms']) / 3, uses_tensor_cores(s, precision), peak,
                                           per_pass - 1),
