@@ -480,7 +480,8 @@ template <int W> struct PairYxSmem {
 // dgemm_mma_body's, so the pass is bit for bit the six-launch one.
 // What bounds the six launches there is the fixed part of each, about 8 us of launch, first loads, a last uneven wave
 // and stores beside 5 to 6 us of products at 96^3; three launches have it half as often and keep every second
-// intermediate out of memory.  Measured, us of a step's first passes, six launches and three: 96^3 303 and 237 (the step
+// intermediate out of memory.  What bounds them are the barriers and dependent waits of the panels (96^3 under ncu: 28 to
+// 30 us a launch, DMMA pipe 37 to 41% of the active cycles, issue 33 to 37%, barrier and wait the first stalls).  Measured, us of a step's first passes, six launches and three: 96^3 303 and 237 (the step
 // 588 and 519), 100 x 100 x 75 349 and 307 (817 and 775), 64 x 64 x 128 (xy and yx by the kernels above) 167 and 140
 // (374 and 346), 128^3 673 and 571.  Two or four panels of 16 in the ring of the six launches' tile GEMM, or skipping
 // its outside fragments, gave nothing (349 to 372 at 100 x 100 x 75).

@@ -1,7 +1,8 @@
 // solver.cu - host side of the B200 cavity solver and its C ABI (cavity_solver.h).
 //
-// One `Solver<T>` owns one cavity: its fields in HBM, a CUDA stream, and two instantiated CUDA graphs of a
-// whole time step (one per state parity, since the step writes the next state into the other buffer set).
+// One `Solver<T>` owns one cavity: its fields in HBM, a CUDA stream, and the instantiated CUDA graphs of a
+// whole time step (one per state parity, since the step writes the next state into the other buffer set; after a stalled
+// solve a second pair with refinement loops).
 // A step is one graph launch: a chain of kernels with one pressure pass per stage (two on the tensor cores), the last
 // block of whose residual decides on the device whether the solve is done; a solve that needs more passes is finished
 // by the host (Solver::settle).  The host waits once per step, to read the control block that holds the clock, the
@@ -225,8 +226,12 @@ public:
         {
             // Mixed form: FDM transforms on the tcgen05 tensor cores (3xTF32) from 128^3 cells up, FP64 DMMA
             // transforms below.  FP32 transforms need two refinement passes where FP64 ones need one, which
-            // only pays once the transforms are large; CAVITY_FDM=tc or =dmma forces either.  The tensor-core
-            // kernel's float4 row loads need nx % 4 == 0.
+            // only pays once the transforms are large; CAVITY_FDM=tc or =dmma forces either.  The line dates from
+            // six launches per pass.  With three the two forms meet lower (us per step, tensor cores and DMMA: 64^3 278
+            // and 191, 64 x 64 x 128 395 and 330, 80^3 380 and 381, 96^3 453 and 493, 112^3 601 and 804, 128 x 128 x 64
+            // 519 and 569, 128^3 800 and 1114; batches of 64 of 64^3 7445 and 5743, 8 of 64 x 64 x 128 2058 and 1769, 4 of
+            // 96^3 1395 and 1702); it has not been moved, and a cavity keeps the arithmetic it had.  The kernels' row
+            // loads need nx % 4 == 0.
             const char* f = std::getenv("CAVITY_FDM");
             const std::string fdm = f ? f : "";
             const bool want = fdm == "tc" || (fdm != "dmma" && n_cell_ >= (1LL << 21));
@@ -1072,7 +1077,9 @@ private:
     // The projection start and the residual of its guess as one launch: for at most 2^18 cells in all (a batch's members
     // together).  Measured against two launches (us per step): 32 x 32 x 8 161 / 173, 32^3 174 / 188, 50 x 50 x 37 201 /
     // 215, 64^3 272 / 282, 64 x 64 x 128 394 / 402; 100 x 100 x 75 FP64 897 / 894, 128^3 960 / 939, 7 x 64^3 997 / 920.
-    // Its chunks do not depend on the batch, so that a member's sums are grouped as those of the cavity alone.
+    // Its chunks do not depend on the batch, so that a member's sums are grouped as those of the cavity alone.  Alone a
+    // cavity would gain to 2^19 cells, but beside others its batch is over the line then and starts in two launches, whose
+    // sums are grouped by other blocks: with the line at 2^19 such a member differed in a last bit from itself alone.
     static constexpr long long kFusedStartCells = 1LL << 18;
     bool fused_start() const { return g_launch_record ? g_batch_fused_start : n_cell_ <= kFusedStartCells; }
     dim3 chunked_grid(long long bpp, int per_sm, int cavities = 0) const {
@@ -1274,9 +1281,9 @@ private:
         check(cudaStreamUpdateCaptureDependencies(stream_, &node, 1, cudaStreamSetCaptureDependencies));
     }
 
-    // The time step for state parity S (backend.cu:877-955), enqueued on stream_: under stream capture (the
-    // refinement loops become conditional while-nodes), or eagerly with the loops driven from the host (the
-    // launch mode for profilers, which cannot see kernels inside graphs that hold conditional nodes).
+    // The time step for state parity S (backend.cu:877-955), enqueued on stream_: under stream capture (a fixed number of
+    // passes, or refinement loops as conditional while-nodes: loops_), or eagerly with the loops driven from the host
+    // (the launch mode for profilers, which see its kernels one by one).
     void enqueue_step(int S, bool timing, bool eager) {
         launch_step_begin(stream_);
         for (int stage = 0; stage < 3; stage++) enqueue_stage(S, stage, timing, eager);
@@ -1448,8 +1455,6 @@ private:
     bool auto_tune_ = false;
     int form_env_ = -1;                 // FP64 pass form named by CAVITY_FDM_FUSED at creation (-1: none)
     int march_per_sm_ = 1;
-    // z-chunks of a march sweep launch: as many as fill the device's resident CTA slots once (all cavities of a
-    // batch together) with at least four layers per chunk; CAVITY_MARCH_CHUNKS overrides
     // Half the height of a column walk's chunk for a launch over these grids (sweep_column.cuh), or 0 where the tile
     // sweep is the faster of the two; their results are the same bit for bit.  The walk's time goes as the layer pairs
     // that an SM walks for the CTAs it runs one after the other (one fits), three of them before each chunk; the tile's
@@ -1508,6 +1513,8 @@ private:
     }
     int column_height() const { return g_launch_record ? g_batch_column : column_height({this}, sms_); }
     int column_env_ = -1;               // CAVITY_COLUMN: 0 the tile, n > 0 the walk in about n z-chunks; -1: the rule
+    // z-chunks of a march sweep launch: as many as fill the device's resident CTA slots once (all cavities of a
+    // batch together) with at least four layers per chunk; CAVITY_MARCH_CHUNKS overrides
     unsigned int march_chunks() const {
         const long long tiles = (long long)((nx_ + kMarchTX - 1) / kMarchTX) * ((ny_ + kMarchTY - 1) / kMarchTY) *
                                 std::max(g_launch_batch, 1);

@@ -25,10 +25,13 @@
 // commit of its MMAs, so copies, splits and MMAs of different panels overlap.  The first basis panels are copied before
 // the previous kernel ends (griddepcontrol): they do not depend on it.
 //
-// Bound: shared memory.  At n = 128 a panel's 12 MMAs read 96 KB of operands (768 clocks at 128 bytes per clock, as
-// long as the MMAs themselves), and 64 KB of splits and copies are written beside them: 1,280 clocks, against about
-// 1,100 that the same loop takes with nothing but its MMAs and barriers.  A launch at 128^3 is one wave of CTAs of
-// 2 x 4 panels; it took 17 us where its two single launches took 28 (the first passes of a step 250 -> 157 us, the step
+// Bound: at 128^3, where a launch is one wave of CTAs of 2 x 4 panels, that chain: the first loads, eight panels and the
+// stores (18 to 23 us under ncu, tensor pipe 13 to 16% of it, shared-memory data pipe 13 to 18%, most stalls on global
+// loads).  With longer rows shared memory: counted at n = 128, a panel's 12 MMAs read 96 KB of operands (768 clocks at 128
+// bytes per clock, as long as the MMAs themselves) and 64 KB of splits and copies are written beside them, 1,280 clocks,
+// where the same loop took 1,000 to 1,150 with nothing but its MMAs and barriers; at 256 x 256 x 64 the plane launches
+// have the tensor pipe busy 27 to 31%.  The inverse holds its potential's values over the products and spills 84 bytes a
+// thread (96 registers are what 18 warps leave), the forward launch 48 with rows beyond 128.  A launch at 128^3 took 17 us where its two single launches took 28 (the first passes of a step 250 -> 157 us, the step
 // 1.086 -> 0.939 ms); at 164 x 164 x 93 the first passes went from 484 to 370 us, at 256^3 from 2,575 to 1,210 us (the
 // step 8.92 -> 6.63 ms).  A pass moves 44 bytes per cell instead of 64.  Splitting the basis here instead (half the
 // bytes to copy, twice the splits) measured slower (164 x 164 x 93: 398 us), as did 8 converting warps (417).
