@@ -99,7 +99,8 @@ long long cavity_estimate_bytes(const CavityConfig* config, int precision);
 
 /* Timing support for benchmarks: run `warmup` untimed steps, then `steps` steps, each bracketed by CUDA
  * events on the solver's stream, with the L2 cache flushed (a 256 MiB device write) before each timed
- * step when flush_l2 != 0.  ms_per_step[steps] receives each step's device time.  When kernel_ms is not NULL,
+ * step when flush_l2 != 0.  ms_per_step[steps] receives each step's device time (of a step that needs more pressure passes
+ * than a queued one holds, to the end of the part that the wait runs).  When kernel_ms is not NULL,
  * `steps` more steps follow through a step graph that also records events around the kernels; kernel_ms[steps]
  * receives the device time of each one's momentum-sweep launches (see also cavity_kernel_times). */
 int cavity_time_steps(CavitySolver* s, int warmup, int steps, int flush_l2, float* ms_per_step, float* kernel_ms);
