@@ -301,6 +301,7 @@ public:
     // queue one step; the parity flips only when it succeeds: sync() checks that for the queued steps
     void queue_step(bool timing) {
         if (pending_.empty()) steps_before_ = hc_.steps;
+        tail_queued_ = false;                    // an earlier step's
         if (eager_) enqueue_step(par_, timing, true);
         else check(cudaGraphLaunch(timing ? texec_[par_] : exec_[loops_][par_], stream_));
         pending_.push_back({par_});

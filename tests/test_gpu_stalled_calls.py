@@ -282,3 +282,19 @@ def test_batch_follows_its_members(monkeypatch):
         calm.close()
         for cav in (stalls, member, alone):
             cav.close()
+
+
+def test_time_steps_behind_queued_steps(monkeypatch):
+    """Steps that do not stall are queued, with their tail, when the timing begins: the wait reads the control block after
+    the timed step, not the tail's earlier copy."""
+    cav, eager = (make('fp64', monkeypatch, eager=e, fdm_rtol=1e-9) for e in (False, True))
+    try:
+        cav.step_async(2)
+        ms = np.zeros(1, dtype=np.float32)
+        cav._call('cavity_time_steps', cav.handle, 0, 1, 0, ms.ctypes.data, None)
+        for _ in range(3):
+            eager.step()
+        assert_same(cav, eager)
+    finally:
+        cav.close()
+        eager.close()
