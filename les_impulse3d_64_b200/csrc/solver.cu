@@ -393,6 +393,7 @@ public:
     void kick(const double* const noise[3], double amp, int passes) override {        // backend.cu:958-978
         probes_fresh_ = false;
         settle_queued();
+        tail_queued_ = false;                    // the control block changes after the tail's copy
         const int S = par_, X2 = par_ ^ 1;
         for (int k = 0; k < 3; k++) {
             const int sx = nx_ + (k == 0), sy = ny_ + (k == 1), sz = nz_ + (k == 2);
@@ -485,6 +486,7 @@ public:
         probes_fresh_ = false;
         if (field < 0 || field > 6) fail("field must be 0..6");
         settle_queued();
+        tail_queued_ = false;                    // the control block changes after the tail's copy
         if (field == 6) {
             check(cudaMemcpyAsync(PHI_[par_], in, sizeof(double) * n_cell_, cudaMemcpyHostToDevice, stream_));
         } else {

@@ -298,3 +298,25 @@ def test_time_steps_behind_queued_steps(monkeypatch):
     finally:
         cav.close()
         eager.close()
+
+
+def test_set_field_while_steps_are_queued(monkeypatch):
+    """A field set behind queued steps clears the potential's history for good: the wait, and a clock set after it, do not
+    bring the steps' back."""
+    queued, eager = (make('fp64', monkeypatch, eager=e, fdm_rtol=1e-9) for e in (False, True))
+    try:
+        queued.step_async(3)
+        for _ in range(3):
+            eager.step()
+        u = 0.9 * eager.field('u')
+        for cav in (queued, eager):
+            cav.set_field('u', u)
+        r = queued.sync()
+        for cav in (queued, eager):
+            cav.set_clock(r['time'], r['steps'], r['dt'])
+            for _ in range(2):
+                cav.step()
+        assert_same(queued, eager)
+    finally:
+        queued.close()
+        eager.close()
